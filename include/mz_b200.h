@@ -333,8 +333,8 @@ enum {
   MZ_K_PREP = 0,    /* coefficients -> knot and evaluation tables          */
   MZ_K_ATOMS,       /* densities, embedding, per-slot reaction vectors      */
   MZ_K_GATHER,      /* per-atom forces, force residuals                     */
-  MZ_K_CELLS,       /* per-cell energy, stress, residual entries            */
-  MZ_K_FINAL,       /* sum of squares + punishments                         */
+  MZ_K_CELLS,       /* per-cell energy, stress, residual entries, objective */
+  MZ_K_FINAL,       /* sum of squares + punishments (moment path)           */
   MZ_K_ADJ,         /* adjoint pass over the neighbour rows                 */
   MZ_K_GRAD_FINAL,  /* table gradient -> coefficient gradient               */
   /* mixed-precision meam/spline over triplet moments (the "FM" path):       */
@@ -344,6 +344,7 @@ enum {
   MZ_K_FM_PRE,      /* adjoint weights, pair-function and U gradients       */
   MZ_K_FM_ADJ,      /* transposed contraction: moment-space gradient        */
   MZ_K_FM_GRAD,     /* moment-space and B-spline gradients -> knot table    */
+  MZ_K_GRAD_SUM,    /* table-gradient partials summed (row kernels)         */
   MZ_NKERNELS
 };
 const char *mz_kernel_name(int kernel);

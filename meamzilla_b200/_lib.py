@@ -133,7 +133,7 @@ _SIGS = {
                                        C.c_void_p]),
 }
 
-MZ_NKERNELS = 13
+MZ_NKERNELS = 14
 
 
 def lib() -> C.CDLL:

@@ -59,7 +59,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)
-    objs = []
+    objs, running = [], []
     common = ["-O3", "-std=c++17", "-I", INCLUDE, "-I", CSRC, "-Xcompiler", "-fPIC,-ffp-contract=off"]
     for src in SOURCES:
         path = os.path.join(CSRC, src)
@@ -70,8 +70,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd += ["-c", path, "-o", obj]
         if verbose:
             print(" ".join(cmd), flush=True)
-        subprocess.run(cmd, check=True)
+        running.append((cmd, subprocess.Popen(cmd)))  # side by side
         objs.append(obj)
+    for cmd, p in running:
+        if p.wait() != 0:
+            raise subprocess.CalledProcessError(p.returncode, cmd)
     tmp = LIB + ".tmp"
     subprocess.run([nvcc()] + ARCH + ["-shared", "-o", tmp] + objs + ["-lcudart"], check=True)
     os.replace(tmp, LIB)

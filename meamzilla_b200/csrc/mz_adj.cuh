@@ -1,7 +1,7 @@
 // Adjoint of the objective with respect to every knot value and end slope.
 //
 // The objective is F = sum of squared residuals.  With the residuals'
-// sensitivities frozen as seeds -- lambda_i = dF/dF_i (k_gather),
+// sensitivities frozen as seeds -- lambda_i = dF/dF_i (k_force),
 // eps_c = dF/dE_atom, mu_c = dF/dS_c, kappa_c = dF/dpen (k_cells) -- the
 // gradient is that of
 //   L = sum_i [eps E_i + kappa pen(rho_i)] + sum_p Lambda_p . V_p
@@ -803,25 +803,49 @@ __global__ void __launch_bounds__(BLOCK_SLOTS, JM || sizeof(R) == 8 ? 2 : (GM ||
   }
 }
 
-// Sum the CTA partials, add the punishment terms, and map the table
-// gradient (y, ypp, end slopes) to the coefficients through the transposed
-// refresh: ypp = M [y; slope_left; slope_right] (Spline3Eq::refresh_basis is
-// linear in them, spline3eq.cpp:192-225).
-__global__ void k_grad_final(DevPot pot, const SplineGeom *__restrict__ geom, const double *__restrict__ tabs,
-                             const double *__restrict__ partial, int nparts, const double *__restrict__ M,
-                             const int *__restrict__ cmap, int P, double *__restrict__ grad) {
+// The partials of every table entry, [ncand][nparts][stride] -> [ncand][stride].
+// 32 entries per CTA; its eight warps take an eighth of the partials each, in
+// order, and the eight sums are added in order.  (One CTA per candidate doing
+// this serially took 70 us for 700 partials of 300 entries; this takes 6.)
+__global__ void __launch_bounds__(256) k_grad_sum(int stride, const double *__restrict__ partial, int nparts,
+                                                  double *__restrict__ sum) {
+  __shared__ double part[8][32];
+  const int c = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+  const int per = (nparts + 7) / 8, b1 = min(nparts, (warp + 1) * per);
+  double s = 0.0;
+  if (e < stride) {
+    const double *p = partial + (size_t)c * nparts * stride + e;
+#pragma unroll 8
+    for (int b = warp * per; b < b1; ++b) s += p[(size_t)b * stride];
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && e < stride) {
+    s = part[0][lane];
+    for (int w = 1; w < 8; ++w) s += part[w][lane];
+    sum[(size_t)c * stride + e] = s;
+  }
+}
+
+// Add the punishment terms to the summed table gradient, and map it
+// (y, ypp, end slopes) to the coefficients through the transposed refresh:
+// ypp = M [y; slope_left; slope_right] (Spline3Eq::refresh_basis is linear in
+// them, spline3eq.cpp:192-225).  One CTA per candidate: a warp per spline, a
+// lane per coefficient, the table and its gradient in shared memory.
+__global__ void __launch_bounds__(256)
+    k_grad_final(DevPot pot, const SplineGeom *__restrict__ geom, const double *__restrict__ tabs,
+                 const double *__restrict__ sum, const double *__restrict__ M, const int *__restrict__ cmap, int P,
+                 double *__restrict__ grad) {
   extern __shared__ double ext[];
   const int c = blockIdx.x;
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int stride = pot.tab_stride;
+  double *tab = ext + stride;
   for (int e = t; e < stride; e += blockDim.x) {
-    double s = 0.0;
-    const double *p = partial + (size_t)c * nparts * stride + e;
-    for (int b = 0; b < nparts; ++b) s += p[(size_t)b * stride];
-    ext[e] = s;
+    ext[e] = sum[(size_t)c * stride + e];
+    tab[e] = tabs[(size_t)c * stride + e];
   }
   __syncthreads();
-  const double *tab = tabs + (size_t)c * stride;
   if (t == 0 && !pot.omit_pen && !pot.pair) {
     if (pot.gmeam) {
       for (int f = 0; f < pot.npair; ++f) {
@@ -853,12 +877,12 @@ __global__ void k_grad_final(DevPot pot, const SplineGeom *__restrict__ geom, co
   }
   __syncthreads();
   double *gc = grad + (size_t)c * P;
-  for (int s = t; s < pot.nsplines; s += blockDim.x) {
+  for (int s = warp; s < pot.nsplines; s += blockDim.x / 32) {
     const SplineGeom g = geom[s];
     const int n = g.n;
     if (g.q5) {
       // spline5eq: (ypp, yp4) = M (y, grad, grad2), M [2n][n+4]
-      for (int col = 0; col < n + 4; ++col) {
+      for (int col = lane; col < n + 4; col += 32) {
         const int te = col < n ? g.toff + col : col < n + 2 ? g.toff + 2 * n + (col - n) : g.toff + 3 * n + 2 + (col - n - 2);
         double acc = ext[te];
         for (int r = 0; r < n; ++r) acc += M[g.moff + r * (n + 4) + col] * ext[g.toff + n + r];
@@ -868,7 +892,7 @@ __global__ void k_grad_final(DevPot pot, const SplineGeom *__restrict__ geom, co
       }
       continue;
     }
-    for (int col = 0; col < n + 2; ++col) {
+    for (int col = lane; col < n + 2; col += 32) {
       double acc = col < n ? ext[g.toff + col] : ext[g.toff + 2 * n + (col - n)];
       for (int r = 0; r < n; ++r) acc += M[g.moff + r * (n + 2) + col] * ext[g.toff + n + r];
       const int ci = col < n ? cmap[g.toff + col] : cmap[g.toff + 2 * n + (col - n)];

@@ -13,17 +13,18 @@
 //             every slot (PotMEAMSpline::fast_compute,
 //             pot_meam_spline.cpp:143-270; PotEAMSpline::fast_compute,
 //             pot_eam_spline.cpp:135-207).
-//   k_gather  one thread per atom: F_i = sum_p V_p(own row) - sum V(incoming
+//   k_force   eight lanes per atom: F_i = sum_p V_p(own row) - sum V(incoming
 //             slots) -- the reference's "atom_j.force -= ..." scatter as a
 //             gather, no atomics.
-//   k_cells   one warp per cell: energy per atom, stress / volume, constraint
+//   k_cells   one CTA per cell: energy per atom, stress / volume, constraint
 //             and the residual vector entries (Potential::accumulate_error,
-//             potential.cpp:415-491).
-//   k_final   one CTA per candidate: sum of squares + style punishments
-//             (pot_meam_spline.cpp:274-278, pot_eam_spline.cpp:211-218).
+//             potential.cpp:415-491); the last CTA of a candidate adds the sum
+//             of squares + style punishments (pot_meam_spline.cpp:274-278,
+//             pot_eam_spline.cpp:211-218).
 // and for the gradient:
 //   k_adj        persistent CTAs over atom blocks, one thread per slot
-//   k_grad_final partial sums, punishment terms, transposed refresh.
+//   k_grad_sum   the CTAs' partial sums
+//   k_grad_final punishment terms, transposed refresh.
 // Forward reductions run in a fixed order (bit-reproducible objective).  The
 // FP64 gradient's table sums are FP64 in a fixed order (bit-reproducible, for
 // any launch variant); the mixed-precision adjoint adds its pair-function and
@@ -73,12 +74,13 @@ struct mz_ctx {
   double *d_params = nullptr, *d_tabs = nullptr, *d_ptabs = nullptr, *d_V = nullptr, *d_aout = nullptr;
   double *d_forces = nullptr, *d_cellobj = nullptr, *d_obj = nullptr, *d_errvec = nullptr;
   double *d_energy = nullptr, *d_stress = nullptr;
-  double *d_aux = nullptr, *d_lam = nullptr, *d_seeds = nullptr, *d_partial = nullptr, *d_grad = nullptr;
+  double *d_aux = nullptr, *d_lam = nullptr, *d_seeds = nullptr, *d_partial = nullptr, *d_grad = nullptr, *d_gsum = nullptr;
+  int *d_count = nullptr;  // k_cells: a candidate's cells done, zero between launches
   float *d_ptabf = nullptr, *d_wtab = nullptr;  // FP32 evaluation tables, g B-spline coefficients
   int *d_err = nullptr;                         // device-side failure flag (bounded waits)
   TcParams tc{};                                // tensor-core forward plan
   bool tc_ok = false;
-  bool q5 = false;  // spline5eq potential: objective only (no adjoint)
+  bool q5 = false;  // a spline5eq spline in the potential
   int nsm = 1;
   // Kernel sequences of the host-buffer entry points captured as CUDA graphs,
   // one per (candidates, precision, outputs); replayed on later calls.
@@ -339,6 +341,22 @@ void smem_attr(K kernel, size_t bytes) {
   ck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attribute");
 }
 
+// The table-gradient partials in d_partial [n][nparts][stride] -> the gradient.
+void launch_grad_final(mz_ctx *ctx, int n, int nparts, double *d_grad) {
+  const double *sum = ctx->d_partial;
+  if (nparts > 1) {
+    Bracket b(ctx, MZ_K_GRAD_SUM);
+    k_grad_sum<<<dim3((ctx->stride + 31) / 32, n), 256, 0, ctx->stream>>>(ctx->stride, ctx->d_partial, nparts,
+                                                                         ctx->d_gsum);
+    ck(cudaGetLastError(), "k_grad_sum launch");
+    sum = ctx->d_gsum;
+  }
+  Bracket b(ctx, MZ_K_GRAD_FINAL);
+  k_grad_final<<<n, 256, 2 * sizeof(double) * ctx->stride, ctx->stream>>>(ctx->pot, ctx->d_geom, ctx->d_tabs, sum,
+                                                                         ctx->d_M, ctx->d_cmap, ctx->P, d_grad);
+  ck(cudaGetLastError(), "k_grad_final launch");
+}
+
 // ------------------------------------------------------- triplet moments
 
 // Candidates per group of the moment path's layouts for a launch of n.
@@ -581,12 +599,7 @@ void enqueue_fm(mz_ctx *ctx, int n, double *d_obj, double *d_errvec, double *d_f
     k_fm_grad<<<n, 256, sm, st>>>(ctx->pot, ctx->d_geom, fp, fp.coef64, ctx->d_partial);
     ck(cudaGetLastError(), "k_fm_grad launch");
   }
-  {
-    Bracket b(ctx, MZ_K_GRAD_FINAL);
-    k_grad_final<<<n, 256, sizeof(double) * ctx->stride, st>>>(ctx->pot, ctx->d_geom, ctx->d_tabs, ctx->d_partial,
-                                                                1, ctx->d_M, ctx->d_cmap, ctx->P, d_grad);
-    ck(cudaGetLastError(), "k_grad_final launch");
-  }
+  launch_grad_final(ctx, n, 1, d_grad);
 }
 
 // Enqueue the objective (and, with d_grad, its gradient) of n candidates
@@ -599,10 +612,9 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
   const bool grad = d_grad != nullptr;
   {
     Bracket b(ctx, MZ_K_PREP);
-    k_prep<<<n, std::max(32, ((ctx->nsplines + 31) / 32) * 32), 0, st>>>(
-        n, ctx->P, d_params, ctx->d_base, ctx->d_cmap, ctx->d_geom, ctx->d_nat, ctx->nsplines, ctx->stride,
-        ctx->d_tabs, ctx->pstride, ctx->d_ptabs, ctx->d_ptabf, ctx->tc_ok ? ctx->d_wtab : nullptr, ctx->pot.s_g,
-        ctx->pot.ntypes, TC_NB, ctx->d_M);
+    prep_launch(n, ctx->P, d_params, ctx->d_base, ctx->d_cmap, ctx->d_geom, ctx->d_nat, ctx->nsplines, ctx->stride,
+                ctx->d_tabs, ctx->pstride, ctx->d_ptabs, ctx->d_ptabf, ctx->tc_ok ? ctx->d_wtab : nullptr,
+                ctx->pot.s_g, ctx->pot.ntypes, TC_NB, ctx->d_M, st);
     ck(cudaGetLastError(), "k_prep launch");
   }
   if (mixed && meam && ctx->fm_on && ctx->fm.ready) {
@@ -634,23 +646,16 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
   }
   {
     Bracket b(ctx, MZ_K_GATHER);
-    dim3 gg((ctx->natoms + 255) / 256, n);
-    k_gather<<<gg, 256, 0, st>>>(ctx->db, ctx->d_V, ctx->d_aout, d_forces, d_errvec, ctx->esize,
-                                 grad ? ctx->d_lam : nullptr);
-    ck(cudaGetLastError(), "k_gather launch");
+    k_force<<<dim3((unsigned)(((int64_t)ctx->natoms * FORCE_LANES + 255) / 256), n), 256, 0, st>>>(
+        ctx->db, ctx->d_V, ctx->d_aout, d_forces, d_errvec, ctx->esize, grad ? ctx->d_lam : nullptr);
+    ck(cudaGetLastError(), "k_force launch");
   }
   {
     Bracket b(ctx, MZ_K_CELLS);
-    dim3 gc((ctx->ncells + 7) / 8, n);
-    k_cells<<<gc, 256, 0, st>>>(ctx->db, ctx->pot, ctx->d_aout, ctx->d_cellobj, d_errvec, ctx->esize, d_energy,
-                                d_stress, grad ? ctx->d_seeds : nullptr);
+    k_cells<<<dim3(ctx->ncells, n), CELL_T, 0, st>>>(ctx->db, ctx->pot, ctx->d_geom, ctx->d_tabs, ctx->d_aout,
+                                                     ctx->d_cellobj, d_obj, d_errvec, ctx->esize, d_energy, d_stress,
+                                                     grad ? ctx->d_seeds : nullptr, ctx->d_count);
     ck(cudaGetLastError(), "k_cells launch");
-  }
-  {
-    Bracket b(ctx, MZ_K_FINAL);
-    k_final<<<n, 256, 0, st>>>(ctx->db, ctx->pot, ctx->d_geom, ctx->d_tabs, ctx->d_cellobj, d_obj, d_errvec,
-                               ctx->esize);
-    ck(cudaGetLastError(), "k_final launch");
   }
   if (!grad) return;
   {
@@ -660,15 +665,10 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
     else mixed ? launch_adj<false, float>(ctx, n, sj) : launch_adj<false, double>(ctx, n, sj);
     ck(cudaGetLastError(), "k_adj launch");
   }
-  {
-    Bracket b(ctx, MZ_K_GRAD_FINAL);
-    // FP64: one partial per group of adj_group blocks; mixed: one per CTA
-    const int nparts = mixed ? ctx->adj_ctas
-                             : (ctx->db.adj_nblocks + ctx->db.adj_group - 1) / std::max(ctx->db.adj_group, 1);
-    k_grad_final<<<n, 256, sizeof(double) * ctx->stride, st>>>(ctx->pot, ctx->d_geom, ctx->d_tabs, ctx->d_partial,
-                                                                nparts, ctx->d_M, ctx->d_cmap, ctx->P, d_grad);
-    ck(cudaGetLastError(), "k_grad_final launch");
-  }
+  // FP64: one partial per group of adj_group blocks; mixed: one per CTA
+  const int nparts = mixed ? ctx->adj_ctas
+                           : (ctx->db.adj_nblocks + ctx->db.adj_group - 1) / std::max(ctx->db.adj_group, 1);
+  launch_grad_final(ctx, n, nparts, d_grad);
 }
 
 // Independent FMA streams: 8 accumulators per thread, no memory traffic.
@@ -1125,6 +1125,11 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
       dp.s_q[m] = m < dp.nj ? pot.spline_index(m == 0 ? G_Q1 : G_Q2, 0) : 0;
     }
     dp.aux_rows = AUX_COUNT * (1 + dp.nj);
+    if (!dp.pair) {
+      const SplineGeom &u0 = geom[dp.s_U], &u1 = geom[dp.s_U + pot.ntypes - 1];
+      dp.u_off = u0.toff;
+      dp.u_len = u1.toff + (u1.q5 ? 3 : 2) * u1.n + (u1.q5 ? 4 : 2) - u0.toff;
+    }
     ctx->npen = style_npen(pot.style, pot.ntypes);
     ctx->esize = style_esize(pot.style, pot.ntypes, db.ncells, db.natoms);
 
@@ -1281,8 +1286,8 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
           fp.NN = NN;
           fp.NB = NBp;
           // the U splines are consecutive in the knot table
-          fp.utoff = im.geom[dp.s_U].toff;
-          fp.ustride = im.geom[dp.s_U + pot.ntypes - 1].toff + 2 * im.geom[dp.s_U + pot.ntypes - 1].n + 2 - fp.utoff;
+          fp.utoff = dp.u_off;
+          fp.ustride = dp.u_len;
           fp.D = pot.ntypes * NA * NN;
           fp.Dpad = (fp.D + FM_DC - 1) / FM_DC * FM_DC;
           fp.nch = fp.Dpad / FM_DC;
@@ -1408,6 +1413,8 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     if (ctx->adj_fits[1]) smem_attr(k_adj<true, float, true, false, true>, ctx->smem_adj[1]);
     if (ctx->adj_fits[0]) smem_attr(k_adj<true, double, false, true, true>, ctx->smem_adj[0]);
     if (ctx->adj_fits[1]) smem_attr(k_adj<true, float, false, true, true>, ctx->smem_adj[1]);
+    if (2 * sizeof(double) * stride > 48 * 1024 && 2 * sizeof(double) * stride <= (size_t)smem_max)
+      smem_attr(k_grad_final, 2 * sizeof(double) * stride);
     int nsm = 0, per_sm = 0;
     ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device), "attribute");
     if (ctx->adj_fits[1])
@@ -1467,8 +1474,9 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     const size_t per_cand =
         sizeof(double) * ((size_t)(3 + (meam ? dp.aux_rows : 0)) * Np + (size_t)(AO_COUNT + 3 + 3) * N +
                           (size_t)ctx->esize + (size_t)(8 + 1 + CS_COUNT) * db.ncells + 2 * (size_t)stride + ctx->pstride +
-                          (size_t)ctx->adj_ctas_max * stride * (1 + ADJ_WARPS) + (size_t)2048 * stride +
-                          2 * (size_t)ctx->P + 1);
+                          (size_t)ctx->adj_ctas_max * stride * (1 + ADJ_WARPS) + (size_t)2049 * stride +
+                          2 * (size_t)ctx->P + 1) +
+        sizeof(int);
     const size_t budget = (size_t)(0.6 * (double)freeb);
     const int cap = (int)std::max<size_t>(1, budget / std::max<size_t>(per_cand, 1));
     ctx->cand_cap = std::min(ctx->max_cand, cap);
@@ -1491,6 +1499,9 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     ctx->d_partial = dalloc<double>(ctx, C * nparts * stride);
     ctx->d_wglob = dalloc<double>(ctx, C * (size_t)ctx->adj_ctas_max * ADJ_WARPS * stride);
     ctx->d_grad = dalloc<double>(ctx, C * ctx->P);
+    ctx->d_gsum = dalloc<double>(ctx, C * stride);
+    ctx->d_count = dalloc<int>(ctx, C);
+    ck(cudaMemset(ctx->d_count, 0, sizeof(int) * C), "count init");
     ctx->d_ptabf = dalloc<float>(ctx, C * ctx->pstride);
     ctx->d_wtab = meam ? dalloc<float>(ctx, C * pot.ntypes * (2 * TC_NB - 1)) : nullptr;
     ctx->d_err = dalloc<int>(ctx, 1);
@@ -1634,9 +1645,9 @@ mz_status mz_gram_device(mz_ctx *ctx, int na, const double *d_a, int64_t lda, in
 }
 
 const char *mz_kernel_name(int k) {
-  static const char *names[MZ_NKERNELS] = {"k_prep",   "k_atoms",      "k_gather",  "k_cells",  "k_final",
+  static const char *names[MZ_NKERNELS] = {"k_prep",   "k_atoms",      "k_force",   "k_cells",  "k_final",
                                            "k_adj",    "k_grad_final", "k_fm_coef", "k_fm_fwd", "k_fm_epi",
-                                           "k_fm_pre", "k_fm_adj",     "k_fm_grad"};
+                                           "k_fm_pre", "k_fm_adj",     "k_fm_grad",    "k_grad_sum"};
   return (k >= 0 && k < MZ_NKERNELS) ? names[k] : "?";
 }
 
@@ -1954,9 +1965,8 @@ extern "C" mz_status mz_objective_noalloc(const mz_db *dbh, const mz_pot *poth, 
            *aout = (double *)D(o_aout), *dforces = (double *)D(o_forces), *cellobj = (double *)D(o_cellobj),
            *dobj = (double *)D(o_obj);
 
-    k_prep<<<1, std::max(32, ((ns + 31) / 32) * 32)>>>(1, P, (const double *)D(o_params), (const double *)D(o_base),
-                                                       (const int *)D(o_cmap), dgeom, (const int *)D(o_nat), ns,
-                                                       stride, tabs, pstride, ptabs);
+    prep_launch(1, P, (const double *)D(o_params), (const double *)D(o_base), (const int *)D(o_cmap), dgeom,
+                (const int *)D(o_nat), ns, stride, tabs, pstride, ptabs, nullptr, nullptr, 0, 0, 0, nullptr, nullptr);
     ck(cudaGetLastError(), "k_prep launch");
     dim3 ga(nblocks, 1);
     if (meam)
@@ -1964,12 +1974,15 @@ extern "C" mz_status mz_objective_noalloc(const mz_db *dbh, const mz_pot *poth, 
     else
       k_atoms<false, double, false><<<ga, BLOCK_SLOTS, sa>>>(d, dp, dgeom, tabs, ptabs, V, aout, nullptr);
     ck(cudaGetLastError(), "k_atoms launch");
-    k_gather<<<dim3((N + 255) / 256, 1), 256>>>(d, V, aout, dforces, nullptr, 0, nullptr);
-    ck(cudaGetLastError(), "k_gather launch");
-    k_cells<<<dim3((NC + 7) / 8, 1), 256>>>(d, dp, aout, cellobj, nullptr, 0, nullptr, nullptr, nullptr);
+    k_force<<<dim3((unsigned)(((int64_t)N * FORCE_LANES + 255) / 256), 1), 256>>>(d, V, aout, dforces, nullptr, 0,
+                                                                                  nullptr);
+    ck(cudaGetLastError(), "k_force launch");
+    // k_cells' counter: the atoms' own-force sums are read by now
+    int *count = reinterpret_cast<int *>(aout);
+    ck(cudaMemset(count, 0, sizeof(int)), "count init");
+    k_cells<<<dim3(NC, 1), CELL_T>>>(d, dp, dgeom, tabs, aout, cellobj, dobj, nullptr, 0, nullptr, nullptr, nullptr,
+                                     count);
     ck(cudaGetLastError(), "k_cells launch");
-    k_final<<<1, 256>>>(d, dp, dgeom, tabs, cellobj, dobj, nullptr, 0);
-    ck(cudaGetLastError(), "k_final launch");
     ck(cudaMemcpy(obj, dobj, sizeof(double), cudaMemcpyDeviceToHost), "cudaMemcpy D2H");
     if (forces) ck(cudaMemcpy(forces, dforces, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost), "cudaMemcpy D2H");
   });

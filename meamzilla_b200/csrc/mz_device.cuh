@@ -89,8 +89,29 @@ struct DevPot {
                       // no embedding, no constraint or punishment entries
   int nj;             // JMEAM direct three-body terms sum p_ij p_ik q_i(cos): 0, 1 or 2
   int s_p[2], s_q[2]; // first spline of p, q (p2, q2)
+  int u_off, u_len;   // the U splines' part of a knot table (consecutive)
   int aux_rows;       // per-slot adjoint sums kept per candidate: 5 (1 + nj)
   double energy_weight, stress_weight;
 };
+
+// Per-atom outputs, [cand][AO_COUNT][natoms].
+enum { AO_AX = 0, AO_AY, AO_AZ, AO_E, AO_S0, AO_PEN = AO_S0 + 6, AO_RHO, AO_FSQ, AO_COUNT };
+// Per-slot triplet sums kept for the adjoint, [cand][aux_rows][npairs]:
+//   G_p = sum_k g f_k,  H_p = sum_k g' f_k cos,  vk_p = sum_k g' f_k u_k,
+// and for each JMEAM term m the same with (q_m, p_m) at rows AUX_COUNT (1 + m) + ...
+enum { AUX_G = 0, AUX_H, AUX_VX, AUX_VY, AUX_VZ, AUX_COUNT };
+// Per-cell adjoint seeds, [cand][CS_COUNT][ncells]: dF/dE_atom, dF/dS (6), dF/dpen.
+enum { CS_EPS = 0, CS_MU0, CS_KAPPA = CS_MU0 + 6, CS_COUNT };
+
+__device__ __forceinline__ int pair_ij_index(int ti, int tj, int nt) {
+  return (ti <= tj) ? ti * nt + tj - (ti * (ti + 1)) / 2 : tj * nt + ti - (tj * (tj + 1)) / 2;
+}
+
+// Share of phi(r_p) in atom i's energy and forces: 1/2 in the double-counted
+// lists; in pair/spline's single list 1, or 1/2 for an image of atom i itself
+// (its two images +n and -n are both listed, pot_pair_spline.cpp:106-113).
+__device__ __forceinline__ double phi_share(const DevPot &pot, bool self) {
+  return pot.pair && !self ? 1.0 : 0.5;
+}
 
 }  // namespace mzb

@@ -5,127 +5,157 @@
 
 namespace mzb {
 
-// Per-atom outputs, [cand][AO_COUNT][natoms].
-enum { AO_AX = 0, AO_AY, AO_AZ, AO_E, AO_S0, AO_PEN = AO_S0 + 6, AO_RHO, AO_FSQ, AO_COUNT };
-// Per-slot triplet sums kept for the adjoint, [cand][aux_rows][npairs]:
-//   G_p = sum_k g f_k,  H_p = sum_k g' f_k cos,  vk_p = sum_k g' f_k u_k,
-// and for each JMEAM term m the same with (q_m, p_m) at rows AUX_COUNT (1 + m) + ...
-enum { AUX_G = 0, AUX_H, AUX_VX, AUX_VY, AUX_VZ, AUX_COUNT };
-// Per-cell adjoint seeds, [cand][CS_COUNT][ncells]: dF/dE_atom, dF/dS (6), dF/dpen.
-enum { CS_EPS = 0, CS_MU0, CS_KAPPA = CS_MU0 + 6, CS_COUNT };
-
 // ------------------------------------------------------------------ k_prep
 
-// Coefficient vectors -> per-candidate knot tables.  cmap has the table's
-// layout: cmap[toff+k] (knot k) and cmap[toff+2n+e] (end e) hold the
-// coefficient index, or -1 where the value is fixed and comes from base.
-__global__ void k_prep(int ncand, int P, const double *__restrict__ params, const double *__restrict__ base,
-                       const int *__restrict__ cmap, const SplineGeom *__restrict__ geom,
-                       const int *__restrict__ nat, int nsplines, int stride, double *__restrict__ tabs,
-                       int pstride, double *__restrict__ ptabs, float *__restrict__ ptabf = nullptr,
-                       float *__restrict__ wtab = nullptr, int s_g = 0, int ng = 0, int nbp = 0,
-                       const double *__restrict__ M = nullptr) {
-  const int c = blockIdx.x;
-  const int s = threadIdx.x;
-  if (c >= ncand || s >= nsplines) return;
-  const SplineGeom g = geom[s];
+// Coefficient vectors -> per-candidate knot tables, one CTA per candidate.
+// cmap has the table's layout: cmap[toff+k] (knot k) and cmap[toff+2n+e]
+// (end e) hold the coefficient index, or -1 where the value is fixed and
+// comes from base.  The work is a few hundred numbers, so only latency
+// counts: the table is gathered by all threads into shared memory, y'' is
+// the refresh matrix M times (y, end slopes), a lane per row, and all threads
+// write the results.  One thread per spline walking global memory through
+// the tridiagonal solve (a serial chain of divisions) took 20 us of a 70 us
+// call (one candidate, 3 splines of 8 to 10 knots); the solve, still a thread
+// per spline but in shared memory, serves callers without M.
+// SM: the table and the solve's scratch fit shared memory (prep_smem);
+// otherwise they stay in global memory (tabs and ptabs hold them).
+__host__ __device__ inline size_t prep_smem(int stride) { return sizeof(double) * 2 * (size_t)stride; }
+
+template <bool SM>
+__global__ void __launch_bounds__(256)
+    k_prep(int P, const double *__restrict__ params, const double *__restrict__ base, const int *__restrict__ cmap,
+           const SplineGeom *__restrict__ geom, const int *__restrict__ nat, int nsplines, int stride,
+           double *__restrict__ tabs, int pstride, double *__restrict__ ptabs, float *__restrict__ ptabf,
+           float *__restrict__ wtab, int s_g, int ng, int nbp, const double *__restrict__ M) {
+  extern __shared__ double psm[];
+  const int c = blockIdx.x, tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const double *pc = params + (size_t)c * P;
-  double *t = tabs + (size_t)c * stride + g.toff;
-  const double *bt = base + g.toff;
-  const int *cm = cmap + g.toff;
-  const int n = g.n;
-  for (int k = 0; k < n; ++k) t[k] = cm[k] >= 0 ? pc[cm[k]] : bt[k];
-  for (int e = 0; e < 2; ++e) t[2 * n + e] = cm[2 * n + e] >= 0 ? pc[cm[2 * n + e]] : bt[2 * n + e];
-  if (g.q5) {
-    // spline5eq: y'' at the ends, then (ypp, yp4) = M (y, grad, grad2) -- the
-    // refresh of Spline5Eq::refresh_basis (spline5eq.cpp:209-293) is linear
-    // in them; M is solved once on the host
-    double *g2 = t + 3 * n + 2, *yp4 = t + 2 * n + 2;
-    for (int e = 0; e < 2; ++e) g2[e] = cm[3 * n + 2 + e] >= 0 ? pc[cm[3 * n + 2 + e]] : bt[3 * n + 2 + e];
-    const double *Ms = M + g.moff;
-    const int nc = n + 4;
-    for (int r = 0; r < 2 * n; ++r) {
-      const double *row = Ms + (size_t)r * nc;
+  double *gtab = tabs + (size_t)c * stride, *gp = ptabs + (size_t)c * pstride;
+  double *tab = SM ? psm : gtab;
+  for (int e = tid; e < stride; e += T) tab[e] = cmap[e] >= 0 ? pc[cmap[e]] : base[e];
+  __syncthreads();
+  for (int s = tid; s < nsplines && !M; s += T) {
+    const SplineGeom g = geom[s];
+    if (g.q5) continue;
+    // Spline3Eq::refresh_basis (spline3eq.cpp:192-225)
+    const int n = g.n;
+    double *y = tab + g.toff, *ypp = y + n;
+    double *u = SM ? psm + stride + g.toff : gp + g.poff;  // n values; the pieces below overwrite them
+    const double inv = g.invstep;
+    const double gl = y[2 * n], gr = y[2 * n + 1];
+    if (nat[2 * s]) {
+      ypp[0] = 0;
+      u[0] = 0;
+    } else {
+      ypp[0] = -0.5;
+      u[0] = (3.0 * inv) * ((y[1] - y[0]) * inv - gl);
+    }
+    for (int i = 1; i < n - 1; ++i) {
+      double p = 0.5 * ypp[i - 1] + 2.0;
+      ypp[i] = (-0.5) / p;
+      double ui = (y[i + 1] - y[i]) * inv - (y[i] - y[i - 1]) * inv;
+      u[i] = (6.0 * ui * 0.5 * inv - 0.5 * u[i - 1]) / p;
+    }
+    double qn, un;
+    if (nat[2 * s + 1]) {
+      qn = un = 0.0;
+    } else {
+      qn = 0.5;
+      un = (3.0 * inv) * (gr - (y[n - 1] - y[n - 2]) * inv);
+    }
+    ypp[n - 1] = (un - qn * u[n - 2]) / (qn * ypp[n - 2] + 1.0);
+    for (int k = n - 2; k >= 0; --k) ypp[k] = ypp[k] * ypp[k + 1] + u[k];
+  }
+  // With M, ypp = M (y, grad) (spline5eq: (ypp, yp4) = M (y, grad, grad2)): the
+  // refreshes (Spline3Eq::refresh_basis, Spline5Eq::refresh_basis,
+  // spline5eq.cpp:209-293) are linear, and M is solved once on the host.  A
+  // warp per spline, a lane per row.
+  for (int s = warp; s < nsplines && M; s += T / 32) {
+    const SplineGeom g = geom[s];
+    const int n = g.n, nc = g.q5 ? n + 4 : n + 2;
+    double *t = tab + g.toff;
+    const double *g2 = t + 3 * n + 2;
+    for (int r = lane; r < (g.q5 ? 2 * n : n); r += 32) {
+      const double *row = M + g.moff + (size_t)r * nc;
       double acc = 0.0;
-      for (int c = 0; c < n; ++c) acc += row[c] * t[c];
-      acc += row[n] * t[2 * n] + row[n + 1] * t[2 * n + 1] + row[n + 2] * g2[0] + row[n + 3] * g2[1];
+#pragma unroll 4
+      for (int q = 0; q < n; ++q) acc += row[q] * t[q];
+      acc += row[n] * t[2 * n] + row[n + 1] * t[2 * n + 1];
+      if (g.q5) acc += row[n + 2] * g2[0] + row[n + 3] * g2[1];
       if (r < n) t[n + r] = acc;
-      else yp4[r - n] = acc;
+      else t[2 * n + 2 + r - n] = acc;
     }
-    double *pc6 = ptabs + (size_t)c * pstride + g.poff;
-    const double H2 = g.step * g.step / 6.0, H4 = g.step * g.step * g.step * g.step / 360.0;
-    for (int k = 0; k < n - 1; ++k) {
-      const double p1 = t[k], p2 = t[k + 1], d21 = t[n + k], d22 = t[n + k + 1], d41 = yp4[k], d42 = yp4[k + 1];
-      double *q = pc6 + 6 * k;
-      q[0] = p1;
-      q[1] = p2 - p1 + H2 * (-2.0 * d21 - d22) + H4 * (8.0 * d41 + 7.0 * d42);
-      q[2] = 3.0 * H2 * d21;
-      q[3] = H2 * (d22 - d21) + H4 * (-20.0 * d41 - 10.0 * d42);
-      q[4] = 15.0 * H4 * d41;
-      q[5] = H4 * (3.0 * d42 - 3.0 * d41);
+  }
+  __syncthreads();
+  if (SM)
+    for (int e = tid; e < stride; e += T) gtab[e] = tab[e];
+  // evaluation tables: the polynomial of every interval in its shift, and
+  // their FP32 copy (mixed precision).  A warp per spline, a lane per interval.
+  for (int s = warp; s < nsplines; s += T / 32) {
+    const SplineGeom g = geom[s];
+    const int n = g.n;
+    const double *y = tab + g.toff, *ypp = y + n;
+    if (g.q5) {
+      const double *yp4 = y + 2 * n + 2;
+      const double H2 = g.step * g.step / 6.0, H4 = g.step * g.step * g.step * g.step / 360.0;
+      for (int k = lane; k < n - 1; k += 32) {
+        const double p1 = y[k], p2 = y[k + 1], d21 = ypp[k], d22 = ypp[k + 1], d41 = yp4[k], d42 = yp4[k + 1];
+        double q[6];
+        q[0] = p1;
+        q[1] = p2 - p1 + H2 * (-2.0 * d21 - d22) + H4 * (8.0 * d41 + 7.0 * d42);
+        q[2] = 3.0 * H2 * d21;
+        q[3] = H2 * (d22 - d21) + H4 * (-20.0 * d41 - 10.0 * d42);
+        q[4] = 15.0 * H4 * d41;
+        q[5] = H4 * (3.0 * d42 - 3.0 * d41);
+        for (int j = 0; j < 6; ++j) {
+          gp[g.poff + 6 * k + j] = q[j];
+          if (ptabf) ptabf[(size_t)c * pstride + g.poff + 6 * k + j] = (float)q[j];
+        }
+      }
+      continue;
     }
-    if (ptabf) {
-      float *pf = ptabf + (size_t)c * pstride + g.poff;
-      for (int k = 0; k < 6 * (n - 1); ++k) pf[k] = (float)pc6[k];
+    const double H = g.step * g.step / 6.0;
+    for (int k = lane; k < n - 1; k += 32) {
+      double q[4];
+      q[0] = y[k];
+      q[1] = y[k + 1] - y[k] - (2.0 * ypp[k] + ypp[k + 1]) * H;
+      q[2] = 3.0 * ypp[k] * H;
+      q[3] = (ypp[k + 1] - ypp[k]) * H;
+      for (int j = 0; j < 4; ++j) {
+        gp[g.poff + 4 * k + j] = q[j];
+        if (ptabf) ptabf[(size_t)c * pstride + g.poff + 4 * k + j] = (float)q[j];
+      }
     }
-    return;
+    if (wtab && lane == 0 && s >= s_g && s < s_g + ng) {
+      // Cubic B-spline coefficients of g on its uniform grid (basis function m
+      // centred on knot m-1): S(x_i) = (w_i + 4 w_i+1 + w_i+2)/6 and
+      // S''(x_i) = (w_i - 2 w_i+1 + w_i+2)/h^2 give w_i+1 = y_i - h^2/6 y''_i,
+      // and the two outer coefficients follow from S'' at the end knots.
+      // Their differences are the coefficients of g' (times h) in the
+      // quadratic B-spline basis; both are stored: [w_0 .. w_nbp-1, dw_0 .. dw_nbp-2].
+      float *w = wtab + ((size_t)c * ng + (s - s_g)) * (2 * nbp - 1);
+      const double h2 = g.step * g.step;
+      double wm[66];
+      for (int i = 0; i < n; ++i) wm[i + 1] = y[i] - h2 / 6.0 * ypp[i];
+      wm[0] = h2 * ypp[0] + 2.0 * wm[1] - wm[2];
+      wm[n + 1] = h2 * ypp[n - 1] + 2.0 * wm[n] - wm[n - 1];
+      for (int i = 0; i < nbp; ++i) w[i] = i < n + 2 ? (float)wm[i] : 0.f;
+      for (int i = 0; i + 1 < nbp; ++i) w[nbp + i] = i + 1 < n + 2 ? (float)(wm[i + 1] - wm[i]) : 0.f;
+    }
   }
-  // Spline3Eq::refresh_basis (spline3eq.cpp:192-225)
-  double u[64];
-  double *y = t, *ypp = t + n;
-  const double inv = g.invstep;
-  const double gl = t[2 * n], gr = t[2 * n + 1];
-  if (nat[2 * s]) {
-    ypp[0] = 0;
-    u[0] = 0;
-  } else {
-    ypp[0] = -0.5;
-    u[0] = (3.0 * inv) * ((y[1] - y[0]) * inv - gl);
-  }
-  for (int i = 1; i < n - 1; ++i) {
-    double p = 0.5 * ypp[i - 1] + 2.0;
-    ypp[i] = (-0.5) / p;
-    double ui = (y[i + 1] - y[i]) * inv - (y[i] - y[i - 1]) * inv;
-    u[i] = (6.0 * ui * 0.5 * inv - 0.5 * u[i - 1]) / p;
-  }
-  double qn, un;
-  if (nat[2 * s + 1]) {
-    qn = un = 0.0;
-  } else {
-    qn = 0.5;
-    un = (3.0 * inv) * (gr - (y[n - 1] - y[n - 2]) * inv);
-  }
-  ypp[n - 1] = (un - qn * u[n - 2]) / (qn * ypp[n - 2] + 1.0);
-  for (int k = n - 2; k >= 0; --k) ypp[k] = ypp[k] * ypp[k + 1] + u[k];
-  // evaluation table: the cubic of every interval in its shift
-  double *pc4 = ptabs + (size_t)c * pstride + g.poff;
-  const double H = g.step * g.step / 6.0;
-  for (int k = 0; k < n - 1; ++k) {
-    pc4[4 * k] = y[k];
-    pc4[4 * k + 1] = y[k + 1] - y[k] - (2.0 * ypp[k] + ypp[k + 1]) * H;
-    pc4[4 * k + 2] = 3.0 * ypp[k] * H;
-    pc4[4 * k + 3] = (ypp[k + 1] - ypp[k]) * H;
-  }
-  if (ptabf) {  // FP32 copy of the evaluation table (mixed precision)
-    float *pf = ptabf + (size_t)c * pstride + g.poff;
-    for (int k = 0; k < 4 * (n - 1); ++k) pf[k] = (float)pc4[k];
-  }
-  if (wtab && s >= s_g && s < s_g + ng) {
-    // Cubic B-spline coefficients of g on its uniform grid (basis function m
-    // centred on knot m-1): S(x_i) = (w_i + 4 w_i+1 + w_i+2)/6 and
-    // S''(x_i) = (w_i - 2 w_i+1 + w_i+2)/h^2 give w_i+1 = y_i - h^2/6 y''_i,
-    // and the two outer coefficients follow from S'' at the end knots.
-    // Their differences are the coefficients of g' (times h) in the
-    // quadratic B-spline basis; both are stored: [w_0 .. w_nbp-1, dw_0 .. dw_nbp-2].
-    float *w = wtab + ((size_t)c * ng + (s - s_g)) * (2 * nbp - 1);
-    const double h2 = g.step * g.step;
-    double wm[66];
-    for (int i = 0; i < n; ++i) wm[i + 1] = y[i] - h2 / 6.0 * ypp[i];
-    wm[0] = h2 * ypp[0] + 2.0 * wm[1] - wm[2];
-    wm[n + 1] = h2 * ypp[n - 1] + 2.0 * wm[n] - wm[n - 1];
-    for (int i = 0; i < nbp; ++i) w[i] = i < n + 2 ? (float)wm[i] : 0.f;
-    for (int i = 0; i + 1 < nbp; ++i) w[nbp + i] = i + 1 < n + 2 ? (float)(wm[i + 1] - wm[i]) : 0.f;
-  }
+}
+
+inline void prep_launch(int ncand, int P, const double *params, const double *base, const int *cmap,
+                        const SplineGeom *geom, const int *nat, int nsplines, int stride, double *tabs, int pstride,
+                        double *ptabs, float *ptabf, float *wtab, int s_g, int ng, int nbp, const double *M,
+                        cudaStream_t st) {
+  const size_t sm = prep_smem(stride);
+  if (sm <= 48 * 1024)
+    k_prep<true><<<ncand, 256, sm, st>>>(P, params, base, cmap, geom, nat, nsplines, stride, tabs, pstride, ptabs,
+                                         ptabf, wtab, s_g, ng, nbp, M);
+  else
+    k_prep<false><<<ncand, 256, 0, st>>>(P, params, base, cmap, geom, nat, nsplines, stride, tabs, pstride, ptabs,
+                                         ptabf, wtab, s_g, ng, nbp, M);
 }
 
 // ----------------------------------------------------------- atom blocks
@@ -153,17 +183,6 @@ __device__ __forceinline__ int slot_owner(const int *a_lo, int na, int t) {
     else hi = mid;
   }
   return lo;
-}
-
-__device__ __forceinline__ int pair_ij_index(int ti, int tj, int nt) {
-  return (ti <= tj) ? ti * nt + tj - (ti * (ti + 1)) / 2 : tj * nt + ti - (tj * (tj + 1)) / 2;
-}
-
-// Share of phi(r_p) in atom i's energy and forces: 1/2 in the double-counted
-// lists; in pair/spline's single list 1, or 1/2 for an image of atom i itself
-// (its two images +n and -n are both listed, pot_pair_spline.cpp:106-113).
-__device__ __forceinline__ double phi_share(const DevPot &pot, bool self) {
-  return pot.pair && !self ? 1.0 : 0.5;
 }
 
 // Pair functions of one slot: phi, rho, f with slopes (pot_meam_spline.cpp:152-191).
@@ -345,7 +364,7 @@ __device__ __forceinline__ void warp_slot_sums(const double *red, int lo, int hi
 //   V_p = u_p (phi'_p/2 + rho'_p U') + U' [u_p (f'_p G_p - f_p H_p / r_p)
 //                                          + f_p vk_p / r_p]
 // is the force atom i's terms add to atom i along slot p; the neighbour
-// receives -V_p (k_gather).  In FP32 the row sums are taken in chunks of 8
+// receives -V_p (k_force).  In FP32 the row sums are taken in chunks of 8
 // terms, each chunk added to an FP64 total.
 template <bool MEAM, typename R, bool AUX, bool GM = false, bool JM = false, bool Q5 = false>
 __global__ void __launch_bounds__(BLOCK_SLOTS, JM ? 2 : sizeof(R) == 4 ? 4 : 3)
@@ -614,83 +633,139 @@ __global__ void __launch_bounds__(BLOCK_SLOTS, JM ? 2 : sizeof(R) == 4 ? 4 : 3)
   }
 }
 
-// ----------------------------------------------------------------- k_gather
+// ------------------------------------------------------------------ k_force
 
 // F_i = sum of V over the atom's own slots - sum of V over the slots whose
 // neighbour is i; then the force residual w (F - F0) (potential.cpp:468-478)
-// and, for the adjoint, lambda_i = dF/dF_i = 2 w e_i.
-__global__ void k_gather(DevDb db, const double *__restrict__ V, double *__restrict__ aout,
-                         double *__restrict__ forces, double *__restrict__ errvec, int esize,
-                         double *__restrict__ lam) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y;
-  const int N = db.natoms;
-  if (i >= N) return;
-  const int64_t Np = db.npairs;
+// and, for the adjoint, lambda_i = dF/dF_i = 2 w e_i.  Eight lanes per atom:
+// a lane per atom walked its 16 to 60 incoming slots one dependent read after
+// another (16 us for 21 k atoms of 16 slots, one candidate; this takes 6).
+constexpr int FORCE_LANES = 8;
+
+__global__ void __launch_bounds__(256)
+    k_force(DevDb db, const double *__restrict__ V, double *__restrict__ aout, double *__restrict__ forces,
+            double *__restrict__ errvec, int esize, double *__restrict__ lam) {
+  const int c = blockIdx.y, N = db.natoms, l = threadIdx.x % FORCE_LANES;
+  const int i0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) / FORCE_LANES), i = min(i0, N - 1);
   double *ao = aout + (size_t)c * AO_COUNT * N;
-  const double *Vc = V + (size_t)c * 3 * Np;  // (x, y, z) per slot: one or two 32-byte sectors a read
-  double fx = ao[AO_AX * N + i], fy = ao[AO_AY * N + i], fz = ao[AO_AZ * N + i];
-  for (int q = db.in_off[i]; q < db.in_off[i + 1]; ++q) {
+  const double *Vc = V + (size_t)c * 3 * db.npairs;  // (x, y, z) per slot: one or two 32-byte sectors a read
+  const int q1 = db.in_off[i + 1], cell = db.atom_cell[i], comp = min(l, 2);
+  const double own = ao[(AO_AX + comp) * N + i], f0 = db.force0[3 * i + comp];
+  double f[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (int q = db.in_off[i] + l; q < q1; q += FORCE_LANES) {
     const double *v = Vc + 3 * (int64_t)db.in_slot[q];
-    fx -= v[0];
-    fy -= v[1];
-    fz -= v[2];
+    f[0] += v[0];
+    f[1] += v[1];
+    f[2] += v[2];
   }
-  const int cell = db.atom_cell[i];
-  const double w = db.cell_w[cell];
-  const double rx = w * (fx - db.force0[3 * i]);
-  const double ry = w * (fy - db.force0[3 * i + 1]);
-  const double rz = w * (fz - db.force0[3 * i + 2]);
-  ao[AO_FSQ * N + i] = rx * rx + ry * ry + rz * rz;
-  if (forces) {
-    double *F = forces + (size_t)c * 3 * N;
-    F[3 * i] = fx;
-    F[3 * i + 1] = fy;
-    F[3 * i + 2] = fz;
-  }
-  if (errvec) {
-    const int a0 = db.cell_atom0[cell];
-    double *e = errvec + (size_t)c * esize + 7 * (cell + 1) + 3 * a0 + 3 * (i - a0);
-    e[0] = rx;
-    e[1] = ry;
-    e[2] = rz;
-  }
-  if (lam) {
-    double *L = lam + (size_t)c * 3 * N;
-    L[i] = 2.0 * w * rx;
-    L[N + i] = 2.0 * w * ry;
-    L[2 * N + i] = 2.0 * w * rz;
+#pragma unroll
+  for (int o = FORCE_LANES / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) f[q] += __shfl_xor_sync(0xffffffffu, f[q], o);
+  // lane l < 3 of the atom: component l
+  const double w = db.cell_w[cell], F = own - (l == 0 ? f[0] : l == 1 ? f[1] : f[2]), r = w * (F - f0);
+  double sq = r * r;
+  sq += __shfl_xor_sync(0xffffffffu, sq, 1);      // lanes 0 and 1: x + y
+  sq += __shfl_down_sync(0xffffffffu, r * r, 2);  // lane 0: + z
+  if (i0 >= N) return;
+  if (l == 0) ao[AO_FSQ * N + i] = sq;
+  if (l < 3) {
+    if (forces) forces[(size_t)c * 3 * N + 3 * i + l] = F;
+    if (errvec) errvec[(size_t)c * esize + 7 * (cell + 1) + 3 * i + l] = r;
+    if (lam) lam[((size_t)c * 3 + l) * N + i] = 2.0 * w * r;
   }
 }
 
 // ------------------------------------------------------------------ k_cells
 
-// One warp per cell (potential.cpp:450-485); with `seeds`, also the adjoint
-// seeds dF/dE_atom, dF/dS_cell and dF/dpen of the cell.
-__global__ void k_cells(DevDb db, DevPot pot, const double *__restrict__ aout, double *__restrict__ cellobj,
-                        double *__restrict__ errvec, int esize, double *__restrict__ energy,
-                        double *__restrict__ stress, double *__restrict__ seeds) {
-  const int cell = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const int lane = threadIdx.x & 31;
-  const int c = blockIdx.y;
-  if (cell >= db.ncells) return;
-  const int N = db.natoms;
+// largest |y| of a spline's knots, by the lanes of a warp
+__device__ __forceinline__ double warp_max_abs_y(const SplineGeom &g, const double *tab, int lane) {
+  double m = 0.0;
+  for (int k = lane; k < g.n; k += 32) m = fmax(m, fabs(tab[g.toff + k]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  return m;
+}
+
+// Sum of the style's punishment entries squared; writes them to ev (may be
+// null).  All lanes of one warp.
+__device__ __forceinline__ double warp_punishments(const DevPot &pot, const SplineGeom *__restrict__ geom,
+                                                   const double *__restrict__ tab, double *ev, int lane) {
+  double total = 0.0;
+  if (pot.pair) return 0.0;  // PotPairSpline::fast_compute, pot_pair_spline.cpp:133
+  const bool meam = pot.style == MZ_STYLE_MEAM_SPLINE || pot.nj > 0;
+  const int npen = pot.gmeam ? pot.npair : meam ? 1 + pot.nj : pot.ntypes;
+  for (int q = 0; q < npen; ++q) {
+    double e = 0.0;
+    if (pot.omit_pen) {
+    } else if (pot.gmeam || meam) {
+      // f-potential magnitude punishment (pot_meam_spline.cpp:274-278), JMEAM's
+      // p (p2) magnitudes (pot_jmeam_spline.cpp:286-299); GMEAM: one per f
+      // spline (pot_gmeam_spline.cpp:173-178)
+      const int s0 = pot.gmeam ? pot.s_f + q : q == 0 ? pot.s_f : pot.s_p[q - 1];
+      const int ns = pot.gmeam ? 1 : pot.npair;
+      double m = 0.0;
+      for (int f = 0; f < ns; ++f) m = fmax(m, warp_max_abs_y(geom[s0 + f], tab, lane));
+      e = 100. * 25. * (1.0 - m) * (1.0 - m);
+    } else {
+      // U'(mid-range) punishment per type (pot_eam_spline.cpp:211-218)
+      const SplineGeom &g = geom[pot.s_U + q];
+      e = 100. * spl_point_any(tab, g, 0.5 * (g.x0 + g.xN)).grad;
+    }
+    total += e * e;
+    if (ev && lane == 0) ev[q] = e;
+  }
+  return total;
+}
+
+// One CTA per cell and candidate: energy per atom, stress / volume, constraint
+// and the residual entries (potential.cpp:450-485), with `seeds` also the
+// adjoint seeds dF/dE_atom, dF/dS_cell and dF/dpen of the cell.  The CTA that
+// counts itself last of a candidate adds the cells' sums of squares in a
+// fixed order, and the style's punishments, into the objective (the work of a
+// launch of its own before: 9 us with one candidate).  count [ncand] is zero
+// at every launch and left zero.  Every sum is in an order that depends on
+// the database alone.  A warp per cell took 27 us on cells of up to 1024
+// atoms (one candidate); a CTA per cell 10.
+constexpr int CELL_T = 128;
+
+__global__ void __launch_bounds__(CELL_T)
+    k_cells(DevDb db, DevPot pot, const SplineGeom *__restrict__ geom, const double *__restrict__ tabs,
+            const double *__restrict__ aout, double *cellobj, double *__restrict__ obj, double *__restrict__ errvec,
+            int esize, double *__restrict__ energy, double *__restrict__ stress, double *__restrict__ seeds,
+            int *count) {
+  __shared__ double part[CELL_T / 32][9];
+  __shared__ double tree[CELL_T];
+  __shared__ int slast;
+  const int cell = blockIdx.x, c = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int N = db.natoms, NC = db.ncells;
   const double *ao = aout + (size_t)c * AO_COUNT * N;
   const int a0 = db.cell_atom0[cell], a1 = db.cell_atom0[cell + 1];
   double v[9];
 #pragma unroll
   for (int q = 0; q < 9; ++q) v[q] = 0.0;
-  for (int a = a0 + lane; a < a1; a += 32) {
+#pragma unroll 2
+  for (int a = a0 + tid; a < a1; a += CELL_T) {
     v[0] += ao[AO_E * N + a];
 #pragma unroll
     for (int q = 0; q < 6; ++q) v[1 + q] += ao[(AO_S0 + q) * N + a];
     v[7] += ao[AO_PEN * N + a];
     v[8] += ao[AO_FSQ * N + a];
   }
+  if (a1 - a0 > 32 * warp) {  // warps past a small cell's atoms have nothing to sum
 #pragma unroll
-  for (int q = 0; q < 9; ++q)
-    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-  if (lane == 0) {
+    for (int q = 0; q < 9; ++q)
+      for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+  }
+  if (lane == 0)
+#pragma unroll
+    for (int q = 0; q < 9; ++q) part[warp][q] = v[q];
+  __syncthreads();
+  if (tid == 0) {
+#pragma unroll
+    for (int q = 0; q < 9; ++q)
+      for (int w = 1; w < CELL_T / 32; ++w) v[q] += part[w][q];
     const int na = a1 - a0;
     const double w = db.cell_w[cell];
     const double E = v[0] / na;
@@ -699,6 +774,7 @@ __global__ void k_cells(DevDb db, DevPot pot, const double *__restrict__ aout, d
     double sum = eE * eE;
     double eS[6], sig[6];
     const double sw = w * db.cell_sw[cell] * pot.stress_weight;
+#pragma unroll
     for (int q = 0; q < 6; ++q) {
       sig[q] = v[1 + q] / db.cell_vol[cell];
       eS[q] = sw * (sig[q] - db.cell_s0[6 * cell + q]);
@@ -707,28 +783,49 @@ __global__ void k_cells(DevDb db, DevPot pot, const double *__restrict__ aout, d
     sum += v[8];
     const double cons = v[7];
     sum += cons * cons;
-    cellobj[(size_t)c * db.ncells + cell] = sum;
+    cellobj[(size_t)c * NC + cell] = sum;
+    __threadfence();
+    slast = atomicAdd(count + c, 1) == NC - 1;
+    if (slast) {
+      __threadfence();
+      count[c] = 0;
+    }
     if (errvec) {
       double *e = errvec + (size_t)c * esize + 7 * cell + 3 * a0;
       e[0] = eE;
       for (int q = 0; q < 6; ++q) e[1 + q] = eS[q];
-      if (!pot.pair) errvec[(size_t)c * esize + 7 * db.ncells + 3 * N + cell] = cons;
+      if (!pot.pair) errvec[(size_t)c * esize + 7 * NC + 3 * N + cell] = cons;
     }
-    if (energy) energy[(size_t)c * db.ncells + cell] = E;
+    if (energy) energy[(size_t)c * NC + cell] = E;
     if (stress)
-      for (int q = 0; q < 6; ++q) stress[((size_t)c * db.ncells + cell) * 6 + q] = sig[q];
+      for (int q = 0; q < 6; ++q) stress[((size_t)c * NC + cell) * 6 + q] = sig[q];
     if (seeds) {
-      double *sd = seeds + (size_t)c * CS_COUNT * db.ncells;
-      sd[CS_EPS * db.ncells + cell] = 2.0 * eE * ew;
-      for (int q = 0; q < 6; ++q) sd[(CS_MU0 + q) * db.ncells + cell] = 2.0 * eS[q] * sw / db.cell_vol[cell];
-      sd[CS_KAPPA * db.ncells + cell] = 2.0 * cons;
+      double *sd = seeds + (size_t)c * CS_COUNT * NC;
+      sd[CS_EPS * NC + cell] = 2.0 * eE * ew;
+      for (int q = 0; q < 6; ++q) sd[(CS_MU0 + q) * NC + cell] = 2.0 * eS[q] * sw / db.cell_vol[cell];
+      sd[CS_KAPPA * NC + cell] = 2.0 * cons;
     }
+  }
+  __syncthreads();
+  if (!slast) return;
+  // ---- the last cell of the candidate: the objective
+  double s = 0.0;
+  for (int i = tid; i < NC; i += CELL_T) s += __ldcg(cellobj + (size_t)c * NC + i);
+  tree[tid] = s;
+  __syncthreads();
+  for (int o = CELL_T / 2; o > 0; o >>= 1) {
+    if (tid < o) tree[tid] += tree[tid + o];
+    __syncthreads();
+  }
+  if (warp == 0) {
+    double *ev = errvec ? errvec + (size_t)c * esize + 8 * NC + 3 * N : nullptr;
+    const double pen = warp_punishments(pot, geom, tabs + (size_t)c * pot.tab_stride, ev, lane);
+    if (lane == 0) obj[c] = tree[0] + pen;
   }
 }
 
 // ------------------------------------------------------------------ k_final
 
-// Sum of squares over cells + the style's punishment entries.
 // Signed largest-|y| knot of one spline (Spline::get_max_y_mag, spline.cpp:58-67).
 __device__ __forceinline__ double spline_max_y(const SplineGeom &g, const double *tab, int *which) {
   double sm = 0.0;
@@ -762,6 +859,8 @@ __device__ __forceinline__ double group_max_y(const DevPot &pot, int s0, const S
   return my;
 }
 
+// The moment path's end (k_fm_cells has the cells' sums): sum of squares over
+// cells + the style's punishment entries.
 __global__ void k_final(DevDb db, DevPot pot, const SplineGeom *__restrict__ geom,
                         const double *__restrict__ tabs, const double *__restrict__ cellobj,
                         double *__restrict__ obj, double *__restrict__ errvec, int esize) {
@@ -776,47 +875,10 @@ __global__ void k_final(DevDb db, DevPot pot, const SplineGeom *__restrict__ geo
     if (t < o) part[t] += part[t + o];
     __syncthreads();
   }
-  if (t == 0) {
-    double total = part[0];
-    const double *tab = tabs + (size_t)c * pot.tab_stride;
+  if (t < 32) {
     double *ev = errvec ? errvec + (size_t)c * esize + 8 * db.ncells + 3 * db.natoms : nullptr;
-    if (pot.pair) {
-      // no punishments (PotPairSpline::fast_compute, pot_pair_spline.cpp:133)
-    } else if (pot.omit_pen) {
-      if (ev) {
-        const int npen = pot.style == MZ_STYLE_MEAM_SPLINE ? 1
-                         : pot.nj > 0                     ? 1 + pot.nj
-                         : pot.gmeam                      ? pot.npair
-                                                          : pot.ntypes;
-        for (int q = 0; q < npen; ++q) ev[q] = 0.0;
-      }
-    } else if (pot.gmeam) {
-      // one f-magnitude punishment per f spline (pot_gmeam_spline.cpp:173-178)
-      for (int f = 0; f < pot.npair; ++f) {
-        const double m = fabs(spline_max_y(geom[pot.s_f + f], tab, nullptr));
-        const double fe = 100. * 25. * (1.0 - m) * (1.0 - m);
-        total += fe * fe;
-        if (ev) ev[f] = fe;
-      }
-    } else if (pot.style == MZ_STYLE_MEAM_SPLINE || pot.nj > 0) {
-      // f-potential magnitude punishment (pot_meam_spline.cpp:274-278), and
-      // JMEAM's p (p2) magnitude punishments (pot_jmeam_spline.cpp:286-299)
-      for (int q = 0; q <= pot.nj; ++q) {
-        const double m = fabs(group_max_y(pot, q == 0 ? pot.s_f : pot.s_p[q - 1], geom, tab, nullptr));
-        const double fe = 100. * 25. * (1.0 - m) * (1.0 - m);
-        total += fe * fe;
-        if (ev) ev[q] = fe;
-      }
-    } else {
-      // U'(mid-range) punishment per type (pot_eam_spline.cpp:211-218)
-      for (int ty = 0; ty < pot.ntypes; ++ty) {
-        const SplineGeom &g = geom[pot.s_U + ty];
-        const double e = 100. * spl_point_any(tab, g, 0.5 * (g.x0 + g.xN)).grad;
-        total += e * e;
-        if (ev) ev[ty] = e;
-      }
-    }
-    obj[c] = total;
+    const double pen = warp_punishments(pot, geom, tabs + (size_t)c * pot.tab_stride, ev, t);
+    if (t == 0) obj[c] = part[0] + pen;
   }
 }
 

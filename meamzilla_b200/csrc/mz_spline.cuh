@@ -189,7 +189,7 @@ __device__ __forceinline__ PointEval spl_point_t(const double *tab, const Spline
   }
   return spl_point(tab, g, r);
 }
-__device__ __noinline__ PointEval spl_point_any(const double *tab, const SplineGeom &g, double r) {
+static __device__ __noinline__ PointEval spl_point_any(const double *tab, const SplineGeom &g, double r) {
   return g.q5 ? spl_point5(tab, g, r) : spl_point(tab, g, r);
 }
 
