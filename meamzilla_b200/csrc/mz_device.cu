@@ -51,6 +51,8 @@
 #include "mz_fm.cuh"
 #include "mz_fm8.cuh"
 #include "mz_gram.cuh"
+#include "mz_rows.cuh"
+#include "mz_rows.hpp"
 
 // ================================================================= context
 
@@ -81,6 +83,10 @@ struct mz_ctx {
   TcParams tc{};                                // tensor-core forward plan
   bool tc_ok = false;
   bool q5 = false;  // a spline5eq spline in the potential
+  // FP64 forward by k_rows (a warp for a few atoms): spline3eq potentials, rows
+  // of up to ROWS_MAXROW slots; else k_atoms
+  bool rows_ok = false;
+  int max_row = 0;
   int nsm = 1;
   // Kernel sequences of the host-buffer entry points captured as CUDA graphs,
   // one per (candidates, precision, outputs); replayed on later calls.
@@ -624,7 +630,11 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
   {
     Bracket b(ctx, MZ_K_ATOMS);
     const size_t sa = ctx->smem_atoms[mixed ? 1 : 0];
-    if (meam && mixed && ctx->tc_ok) {
+    if (!mixed && ctx->rows_ok) {
+      RowsForward a{ctx->db,     ctx->pot,    meam,         ctx->max_row, n, ctx->nsm, ctx->d_geom, ctx->d_tabs,
+                    ctx->d_ptabs, ctx->d_V,   ctx->d_aout,  grad && meam ? ctx->d_aux : nullptr, st};
+      ck(rows_forward(a), "k_rows launch");
+    } else if (meam && mixed && ctx->tc_ok) {
       dim3 gt(std::min(ctx->nsm, ctx->natoms), (n + TC_CANDS - 1) / TC_CANDS);
       const size_t st_bytes = (size_t)ctx->tc.smem_bytes;
       if (grad)
@@ -802,6 +812,67 @@ int packed_knots(const Db &db, int64_t s) {
   return (db.pair_knot[nf * s] + 1) | ((db.pair_knot[nf * s + 1] + 1) << 8) | ((db.pair_knot[nf * s + 2] + 1) << 16) |
          (nf > 3 ? (db.pair_knot[nf * s + 3] + 1) << 24 : 0);
 }
+
+// The per-slot arrays of DevDb from the database's own (unit vectors (x, y, z)
+// per slot, shifts and knots [Np][nf]).
+struct PairLayout {
+  double *u[3], *shift;
+  float *f[4], *shiftf;  // u_x, u_y, u_z, r
+  int *knot;
+  signed char *knot_p2;
+  double2 *pair2;  // null: not wanted
+  int2 *meta;
+};
+__global__ void __launch_bounds__(256)
+    k_pair_layout(int64_t Np, int nf, const double *__restrict__ r, const double *__restrict__ u,
+                  const double *__restrict__ shift, const signed char *__restrict__ knot, const int *__restrict__ nbr,
+                  const int *__restrict__ type, PairLayout o) {
+  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= Np) return;
+  const double x = u[3 * s], y = u[3 * s + 1], z = u[3 * s + 2], rr = r[s];
+  o.u[0][s] = x;
+  o.u[1][s] = y;
+  o.u[2][s] = z;
+  o.f[0][s] = (float)x;
+  o.f[1][s] = (float)y;
+  o.f[2][s] = (float)z;
+  o.f[3][s] = (float)rr;
+  for (int q = 0; q < nf; ++q) {
+    const double b = shift[nf * s + q];
+    o.shift[q * Np + s] = b;
+    o.shiftf[q * Np + s] = (float)b;
+  }
+  const signed char *k = knot + nf * s;
+  const int kn = (k[0] + 1) | ((k[1] + 1) << 8) | ((k[2] + 1) << 16) | (nf > 3 ? (k[3] + 1) << 24 : 0);
+  o.knot[s] = kn;
+  if (o.knot_p2) o.knot_p2[s] = k[4];
+  if (o.pair2) {
+    o.pair2[s] = make_double2(x, y);
+    o.pair2[Np + s] = make_double2(z, rr);
+    o.pair2[2 * Np + s] = make_double2(1.0 / rr, shift[nf * s + 2]);
+    o.pair2[3 * Np + s] = make_double2(shift[nf * s], shift[nf * s + 1]);
+    o.meta[s] = make_int2(kn, type[nbr[s]]);
+  }
+}
+
+// Device buffers that live for one block of code.
+struct Scratch {
+  std::vector<void *> p;
+  template <class T>
+  const T *upload(const T *h, size_t n) {
+    void *d = nullptr;
+    const cudaError_t e = cudaMalloc(&d, std::max<size_t>(1, n) * sizeof(T));
+    if (e != cudaSuccess)
+      throw Failure{MZ_ERR_NOMEM, std::string("device allocation of ") + std::to_string(n * sizeof(T)) +
+                                      " bytes failed: " + cudaGetErrorString(e)};
+    p.push_back(d);
+    if (n) ck(cudaMemcpy(d, h, n * sizeof(T), cudaMemcpyHostToDevice), "cudaMemcpy H2D");
+    return static_cast<const T *>(d);
+  }
+  ~Scratch() {
+    for (void *d : p) cudaFree(d);
+  }
+};
 
 // ---------------------------------------------------------------- autotuner
 
@@ -1125,6 +1196,17 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
       dp.s_q[m] = m < dp.nj ? pot.spline_index(m == 0 ? G_Q1 : G_Q2, 0) : 0;
     }
     dp.aux_rows = AUX_COUNT * (1 + dp.nj);
+    dp.ang_cover = 1;
+    if (meam) {
+      dp.ang_p0 = geom[dp.s_g].poff / 4;
+      auto covers = [&](int s0, int count) {
+        for (int s = s0; s < s0 + count; ++s)
+          if (geom[s].x0 - 0.9 * geom[s].step > -1.0 || geom[s].xN + 0.9 * geom[s].step < 1.0 || geom[s].cut < 1.0 + 1e-9)
+            dp.ang_cover = 0;
+      };
+      covers(dp.s_g, dp.gmeam ? pot.ntypes * dp.npair : pot.ntypes);
+      for (int m = 0; m < dp.nj; ++m) covers(dp.s_q[m], pot.ntypes);
+    }
     if (!dp.pair) {
       const SplineGeom &u0 = geom[dp.s_U], &u1 = geom[dp.s_U + pot.ntypes - 1];
       dp.u_off = u0.toff;
@@ -1151,50 +1233,54 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     d.atom_cell = dupload(ctx, db.atom_cell.data(), db.atom_cell.size());
     d.force0 = dupload(ctx, db.atom_force0.data(), db.atom_force0.size());
     const int nf = db.nfun;
-    std::vector<int> off32(N + 1), inoff32(N + 1), inslot32(Np), knot32(Np);
-    std::vector<signed char> knotp2(nf > 4 ? Np : 0);
+    std::vector<int> off32(N + 1), inoff32(N + 1), inslot32(Np);
     for (int i = 0; i <= N; ++i) {
       off32[i] = (int)db.pair_off[i];
       inoff32[i] = (int)db.in_off[i];
     }
-    for (int64_t s = 0; s < Np; ++s) {
-      inslot32[s] = (int)db.in_slot[s];
-      knot32[s] = packed_knots(db, s);
-      if (nf > 4) knotp2[s] = db.pair_knot[nf * s + 4];
-    }
-    d.pair_knot_p2 = nf > 4 ? dupload(ctx, knotp2.data(), knotp2.size()) : nullptr;
+    for (int64_t s = 0; s < Np; ++s) inslot32[s] = (int)db.in_slot[s];
     d.pair_off = dupload(ctx, off32.data(), off32.size());
     d.in_off = dupload(ctx, inoff32.data(), inoff32.size());
     d.in_slot = dupload(ctx, inslot32.data(), inslot32.size());
-    d.pair_knot = dupload(ctx, knot32.data(), knot32.size());
     d.pair_nbr = dupload(ctx, db.pair_nbr.data(), db.pair_nbr.size());
-    {
-      std::vector<double> ux(Np), uy(Np), uz(Np), sh(nf * Np);
-      std::vector<float> rf(Np), uxf(Np), uyf(Np), uzf(Np), shf(nf * Np);
-      for (int64_t s = 0; s < Np; ++s) {
-        ux[s] = db.pair_u[3 * s];
-        uy[s] = db.pair_u[3 * s + 1];
-        uz[s] = db.pair_u[3 * s + 2];
-        rf[s] = (float)db.pair_r[s];
-        uxf[s] = (float)ux[s];
-        uyf[s] = (float)uy[s];
-        uzf[s] = (float)uz[s];
-        for (int q = 0; q < nf; ++q) {
-          sh[q * Np + s] = db.pair_shift[nf * s + q];
-          shf[q * Np + s] = (float)db.pair_shift[nf * s + q];
-        }
-      }
-      d.pair_r = dupload(ctx, db.pair_r.data(), Np);
-      d.pair_ux = dupload(ctx, ux.data(), Np);
-      d.pair_uy = dupload(ctx, uy.data(), Np);
-      d.pair_uz = dupload(ctx, uz.data(), Np);
-      d.pair_shift = dupload(ctx, sh.data(), nf * Np);
-      d.pair_rf = dupload(ctx, rf.data(), Np);
-      d.pair_uxf = dupload(ctx, uxf.data(), Np);
-      d.pair_uyf = dupload(ctx, uyf.data(), Np);
-      d.pair_uzf = dupload(ctx, uzf.data(), Np);
-      d.pair_shiftf = dupload(ctx, shf.data(), nf * Np);
+    d.pair_r = dupload(ctx, db.pair_r.data(), Np);
+    // every other per-slot array, laid out on the device from the database's
+    PairLayout pl{};
+    pl.u[0] = dalloc<double>(ctx, Np);
+    pl.u[1] = dalloc<double>(ctx, Np);
+    pl.u[2] = dalloc<double>(ctx, Np);
+    for (int q = 0; q < 4; ++q) pl.f[q] = dalloc<float>(ctx, Np);
+    pl.shift = dalloc<double>(ctx, nf * Np);
+    pl.shiftf = dalloc<float>(ctx, nf * Np);
+    pl.knot = dalloc<int>(ctx, Np);
+    pl.knot_p2 = nf > 4 ? dalloc<signed char>(ctx, Np) : nullptr;
+    if (!ctx->q5 && rows_lpa(db.max_row) > 0) {
+      pl.pair2 = dalloc<double2>(ctx, 4 * Np);
+      pl.meta = dalloc<int2>(ctx, Np);
     }
+    {
+      Scratch raw;
+      const double *h_u = raw.upload(db.pair_u.data(), 3 * Np), *h_shift = raw.upload(db.pair_shift.data(), nf * Np);
+      const signed char *h_knot = raw.upload(reinterpret_cast<const signed char *>(db.pair_knot.data()), nf * Np);
+      if (Np > 0)
+        k_pair_layout<<<(unsigned)((Np + 255) / 256), 256, 0, ctx->stream>>>(Np, nf, d.pair_r, h_u, h_shift, h_knot,
+                                                                            d.pair_nbr, d.atom_type, pl);
+      ck(cudaGetLastError(), "k_pair_layout launch");
+      ck(cudaStreamSynchronize(ctx->stream), "pair layout");
+    }
+    d.pair_ux = pl.u[0];
+    d.pair_uy = pl.u[1];
+    d.pair_uz = pl.u[2];
+    d.pair_uxf = pl.f[0];
+    d.pair_uyf = pl.f[1];
+    d.pair_uzf = pl.f[2];
+    d.pair_rf = pl.f[3];
+    d.pair_shift = pl.shift;
+    d.pair_shiftf = pl.shiftf;
+    d.pair_knot = pl.knot;
+    d.pair_knot_p2 = pl.knot_p2;
+    d.pair2 = pl.pair2;
+    d.pair_meta = pl.meta;
     // atom blocks: consecutive atoms, <= cap slots and <= cap / 4 atoms, for
     // each of the autotuner's caps (a row longer than the cap is a block of its own)
     for (int v = 0; v < mz_ctx::NCAPS; ++v) {
@@ -1354,6 +1440,9 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     int smem_max = 0;
     ck(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device), "attribute");
     ctx->smem_optin = smem_max;
+    ctx->max_row = db.max_row;
+    ctx->rows_ok = !ctx->q5 && rows_lpa(db.max_row) > 0 &&
+                   rows_forward_bytes(dp, rows_lpa(db.max_row)) <= (size_t)smem_max;
     if (ctx->smem_atoms[0] > (size_t)smem_max)
       throw Failure{MZ_ERR_RANGE, "potential too large for the kernels' shared-memory tables"};
     // the gradient of a precision whose adjoint tables do not fit is refused at the call

@@ -53,6 +53,9 @@ struct DevDb {
   const int *pair_knot;           // packed: (phi+1) | (rho+1) << 8 | (f+1) << 16 | (p+1) << 24
   const signed char *pair_knot_p2;  // JMEAM2: knot of p2 (-1: none), else null
   const float *pair_rf, *pair_uxf, *pair_uyf, *pair_uzf, *pair_shiftf;  // FP32 copies
+  // the FP64 row kernels' copy: 16-byte loads, consecutive slots contiguous
+  const double2 *pair2;           // [4][Np] (u_x, u_y), (u_z, r), (1 / r, f's shift), (phi's, rho's shift)
+  const int2 *pair_meta;          // [Np] packed knots, type of the neighbour
   // atom blocks
   const int *blk_atom0;           // [nblocks+1]
   // atom blocks of the adjoint: atoms grouped by type (adj_atoms, a
@@ -89,6 +92,8 @@ struct DevPot {
                       // no embedding, no constraint or punishment entries
   int nj;             // JMEAM direct three-body terms sum p_ij p_ik q_i(cos): 0, 1 or 2
   int s_p[2], s_q[2]; // first spline of p, q (p2, q2)
+  int ang_cover;      // every angular spline's knots reach (nearly) over [-1, 1] (see mz_rows.cuh)
+  int ang_p0;         // first piece of the first g spline
   int u_off, u_len;   // the U splines' part of a knot table (consecutive)
   int aux_rows;       // per-slot adjoint sums kept per candidate: 5 (1 + nj)
   double energy_weight, stress_weight;
