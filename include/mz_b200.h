@@ -345,6 +345,7 @@ enum {
   MZ_K_FM_ADJ,      /* transposed contraction: moment-space gradient        */
   MZ_K_FM_GRAD,     /* moment-space and B-spline gradients -> knot table    */
   MZ_K_GRAD_SUM,    /* table-gradient partials summed (row kernels)         */
+  MZ_K_RADIAL,      /* radial functions' gradient sums (FP64 row kernels)   */
   MZ_NKERNELS
 };
 const char *mz_kernel_name(int kernel);

@@ -133,7 +133,7 @@ _SIGS = {
                                        C.c_void_p]),
 }
 
-MZ_NKERNELS = 14
+MZ_NKERNELS = 15
 
 
 def lib() -> C.CDLL:

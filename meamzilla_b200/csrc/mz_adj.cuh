@@ -16,12 +16,15 @@
 // JMEAM's terms sum p_j p_k q(cos) enter E_i directly and V_p without U':
 // each is the g channel with (chi, U', f, g) replaced by (eps, 1, p, q) and
 // runs as one more pass over the row with the same shared-memory rows.
+// FP64 gradients without such terms, of spline3eq potentials and rows of up to
+// 128 slots, run in mz_rows_adj.cuh instead.
 #pragma once
 
 #include <type_traits>
 
 #include "mz_fwd.cuh"
 #include "mz_fwd2.cuh"
+#include "mz_rows.hpp"
 
 namespace mzb {
 
@@ -803,49 +806,45 @@ __global__ void __launch_bounds__(BLOCK_SLOTS, JM || sizeof(R) == 8 ? 2 : (GM ||
   }
 }
 
-// The partials of every table entry, [ncand][nparts][stride] -> [ncand][stride].
-// 32 entries per CTA; its eight warps take an eighth of the partials each, in
-// order, and the eight sums are added in order.  (One CTA per candidate doing
-// this serially took 70 us for 700 partials of 300 entries; this takes 6.)
-__global__ void __launch_bounds__(256) k_grad_sum(int stride, const double *__restrict__ partial, int nparts,
-                                                  double *__restrict__ sum) {
-  __shared__ double part[8][32];
-  const int c = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
-  const int per = (nparts + 7) / 8, b1 = min(nparts, (warp + 1) * per);
+// The partials of up to two sets of sums, [ncand][nparts][len] -> [ncand][len].
+// 32 sums per CTA; its 32 warps take a run of the partials each, in order, and
+// the runs' sums are added in order.  (One CTA per candidate doing this
+// serially took 70 us for 700 partials of 300 sums; this takes 5.)
+struct GradSums {
+  const double *partial[2];
+  double *sum[2];
+  int nparts[2], len[2];
+};
+__global__ void __launch_bounds__(1024) k_grad_sum(GradSums g) {
+  __shared__ double part[32][33];
+  const int blocks0 = (g.len[0] + 31) / 32, set = (int)blockIdx.x < blocks0 ? 0 : 1;
+  const int c = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e0 = 32 * ((int)blockIdx.x - (set ? blocks0 : 0)), e = e0 + lane, nparts = g.nparts[set], len = g.len[set];
+  const int per = (nparts + 31) / 32, b1 = min(nparts, (warp + 1) * per);
   double s = 0.0;
-  if (e < stride) {
-    const double *p = partial + (size_t)c * nparts * stride + e;
-#pragma unroll 8
-    for (int b = warp * per; b < b1; ++b) s += p[(size_t)b * stride];
+  if (e < len) {
+    const double *p = g.partial[set] + (size_t)c * nparts * len + e;
+#pragma unroll 16
+    for (int b = warp * per; b < b1; ++b) s += p[(size_t)b * len];
   }
   part[warp][lane] = s;
   __syncthreads();
-  if (warp == 0 && e < stride) {
-    s = part[0][lane];
-    for (int w = 1; w < 8; ++w) s += part[w][lane];
-    sum[(size_t)c * stride + e] = s;
-  }
+  // lane w of warp q holds run w of sum q: a fixed tree
+  s = part[lane][warp];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0 && e0 + warp < len) g.sum[set][(size_t)c * len + e0 + warp] = s;
 }
 
-// Add the punishment terms to the summed table gradient, and map it
+// Add the punishment terms to the table gradient ext, and map it
 // (y, ypp, end slopes) to the coefficients through the transposed refresh:
 // ypp = M [y; slope_left; slope_right] (Spline3Eq::refresh_basis is linear in
 // them, spline3eq.cpp:192-225).  One CTA per candidate: a warp per spline, a
 // lane per coefficient, the table and its gradient in shared memory.
-__global__ void __launch_bounds__(256)
-    k_grad_final(DevPot pot, const SplineGeom *__restrict__ geom, const double *__restrict__ tabs,
-                 const double *__restrict__ sum, const double *__restrict__ M, const int *__restrict__ cmap, int P,
-                 double *__restrict__ grad) {
-  extern __shared__ double ext[];
-  const int c = blockIdx.x;
+__device__ __forceinline__ void grad_finish(const DevPot &pot, const SplineGeom *__restrict__ geom, double *ext,
+                                            const double *tab, const double *__restrict__ M,
+                                            const int *__restrict__ cmap, double *__restrict__ gc) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int stride = pot.tab_stride;
-  double *tab = ext + stride;
-  for (int e = t; e < stride; e += blockDim.x) {
-    ext[e] = sum[(size_t)c * stride + e];
-    tab[e] = tabs[(size_t)c * stride + e];
-  }
-  __syncthreads();
   if (t == 0 && !pot.omit_pen && !pot.pair) {
     if (pot.gmeam) {
       for (int f = 0; f < pot.npair; ++f) {
@@ -876,7 +875,6 @@ __global__ void __launch_bounds__(256)
     }
   }
   __syncthreads();
-  double *gc = grad + (size_t)c * P;
   for (int s = warp; s < pot.nsplines; s += blockDim.x / 32) {
     const SplineGeom g = geom[s];
     const int n = g.n;
@@ -899,6 +897,37 @@ __global__ void __launch_bounds__(256)
       if (ci >= 0) gc[ci] = acc;
     }
   }
+}
+
+__global__ void __launch_bounds__(256)
+    k_grad_final(DevPot pot, const SplineGeom *__restrict__ geom, const double *__restrict__ tabs,
+                 const double *__restrict__ sum, const double *__restrict__ M, const int *__restrict__ cmap, int P,
+                 double *__restrict__ grad) {
+  extern __shared__ double ext[];
+  const int c = blockIdx.x, stride = pot.tab_stride;
+  double *tab = ext + stride;
+  for (int e = threadIdx.x; e < stride; e += blockDim.x) {
+    ext[e] = sum[(size_t)c * stride + e];
+    tab[e] = tabs[(size_t)c * stride + e];
+  }
+  __syncthreads();
+  grad_finish(pot, geom, ext, tab, M, cmap, grad + (size_t)c * P);
+}
+
+// The same from the row adjoint's sums: angular pieces and U tables
+// [ncand][4 nang + u_len], radial pieces [ncand][4 nb].
+__global__ void __launch_bounds__(256)
+    k_rows_grad_final(DevPot pot, RadialPlan R, int nang, const SplineGeom *__restrict__ geom,
+                      const double *__restrict__ tabs, const double *__restrict__ ang, const double *__restrict__ rad,
+                      const double *__restrict__ M, const int *__restrict__ cmap, int P, double *__restrict__ grad) {
+  extern __shared__ double ext[];
+  const int c = blockIdx.x, stride = pot.tab_stride;
+  double *tab = ext + stride;
+  for (int e = threadIdx.x; e < stride; e += blockDim.x) tab[e] = tabs[(size_t)c * stride + e];
+  rows_pieces_to_table(pot, geom, R, nang, pot.ang_p0, ang + (size_t)c * (4 * nang + pot.u_len),
+                       rad + (size_t)c * 4 * R.nb, ext);
+  __syncthreads();
+  grad_finish(pot, geom, ext, tab, M, cmap, grad + (size_t)c * P);
 }
 
 }  // namespace mzb

@@ -44,6 +44,7 @@
 #include "mz_b200.h"
 #include "mz_device.cuh"
 #include "mz_host.hpp"
+#include "mz_rows.hpp"
 #include "mz_adj.cuh"
 #include "mz_fwd2.cuh"
 #include "mz_adj2.cuh"
@@ -52,7 +53,6 @@
 #include "mz_fm8.cuh"
 #include "mz_gram.cuh"
 #include "mz_rows.cuh"
-#include "mz_rows.hpp"
 
 // ================================================================= context
 
@@ -87,6 +87,16 @@ struct mz_ctx {
   // of up to ROWS_MAXROW slots; else k_atoms
   bool rows_ok = false;
   int max_row = 0;
+  // and the FP64 adjoint by k_rows_adj (not for JMEAM's direct terms); else k_adj
+  struct Radj {
+    bool ready = false, failed = false;
+    RowsAdjoint args{};
+    int len = 0, nang = 0;          // a warp's partial, angular pieces
+    double *sum = nullptr, *rsum = nullptr;
+  } radj;
+  int radial_nint[3] = {0, 0, 0};   // most intervals of a phi, rho, f spline
+  std::vector<int4> adj_order;      // the adjoint's atom order: (atom, first slot, slots | type << 16, cell)
+  size_t wglob_len = 0;             // doubles of d_wglob
   int nsm = 1;
   // Kernel sequences of the host-buffer entry points captured as CUDA graphs,
   // one per (candidates, precision, outputs); replayed on later calls.
@@ -347,20 +357,150 @@ void smem_attr(K kernel, size_t bytes) {
   ck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attribute");
 }
 
+void launch_grad_sum(mz_ctx *ctx, int n, const GradSums &g) {
+  Bracket b(ctx, MZ_K_GRAD_SUM);
+  k_grad_sum<<<dim3((g.len[0] + 31) / 32 + (g.len[1] + 31) / 32, n), 1024, 0, ctx->stream>>>(g);
+  ck(cudaGetLastError(), "k_grad_sum launch");
+}
+
 // The table-gradient partials in d_partial [n][nparts][stride] -> the gradient.
 void launch_grad_final(mz_ctx *ctx, int n, int nparts, double *d_grad) {
   const double *sum = ctx->d_partial;
   if (nparts > 1) {
-    Bracket b(ctx, MZ_K_GRAD_SUM);
-    k_grad_sum<<<dim3((ctx->stride + 31) / 32, n), 256, 0, ctx->stream>>>(ctx->stride, ctx->d_partial, nparts,
-                                                                         ctx->d_gsum);
-    ck(cudaGetLastError(), "k_grad_sum launch");
+    GradSums g{};
+    g.partial[0] = ctx->d_partial;
+    g.sum[0] = ctx->d_gsum;
+    g.nparts[0] = nparts;
+    g.len[0] = ctx->stride;
+    launch_grad_sum(ctx, n, g);
     sum = ctx->d_gsum;
   }
   Bracket b(ctx, MZ_K_GRAD_FINAL);
   k_grad_final<<<n, 256, 2 * sizeof(double) * ctx->stride, ctx->stream>>>(ctx->pot, ctx->d_geom, ctx->d_tabs, sum,
                                                                          ctx->d_M, ctx->d_cmap, ctx->P, d_grad);
   ck(cudaGetLastError(), "k_grad_final launch");
+}
+
+// The FP64 row adjoint's plan (groups of atoms, slots by radial interval) and
+// its partials' buffers, at the first FP64 gradient.  False where it does not
+// apply or its memory is not there: k_adj then.
+bool rows_adj_prepare(mz_ctx *ctx) {
+  auto &ra = ctx->radj;
+  if (ra.ready) return true;
+  if (ra.failed || !ctx->rows_ok || ctx->pot.nj > 0) return false;
+  const bool meam = style_meam(ctx->pot.style);
+  const int N = ctx->natoms;
+  const size_t C = ctx->cand_cap, Np = ctx->npairs;
+  const size_t mark = ctx->allocs.size();
+  try {
+    RowsAdjoint &a = ra.args;
+    a.db = ctx->db;
+    a.pot = ctx->pot;
+    a.meam = meam;
+    a.max_row = ctx->max_row;
+    RadialPlan &R = a.radial;
+    R = RadialPlan{};
+    R.nfun = meam ? 3 : ctx->pot.pair ? 1 : 2;
+    const int counts[3] = {ctx->pot.npair, ctx->pot.ntypes, ctx->pot.npair};
+    for (int F = 0; F < R.nfun; ++F) {
+      R.nint[F] = ctx->radial_nint[F];
+      R.b0[F + 1] = R.b0[F] + counts[F] * R.nint[F];
+    }
+    R.nb = R.b0[R.nfun];
+    // one wave of segments (4 CTAs per SM) while that keeps them short
+    R.seg = (int)std::min<size_t>(RADIAL_SEG, std::max<size_t>(256, (Np + 4 * ctx->nsm - 1) / (4 * ctx->nsm)));
+    R.seg = (R.seg + 31) & ~31;
+    R.nseg = (int)((Np + R.seg - 1) / R.seg);
+    int smem_sm = 0;
+    ck(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device), "attribute");
+    const RowsAdjShape sh = rows_adj_shape(ctx->pot, a.max_row, meam, ctx->smem_optin, smem_sm);
+    if (R.nb > RADIAL_MAXB || sh.warps == 0) {
+      ra.failed = true;
+      return false;
+    }
+    // groups of atoms of one type
+    const int aw = 32 / rows_adj_lpa(a.max_row);
+    std::vector<int4> desc;
+    desc.reserve((size_t)N + 64);
+    for (int q = 0, first = 0; q < N; ++q) {
+      const int4 e = ctx->adj_order[q];
+      if (q > 0 && (q - first == aw || (e.z >> 16) != (ctx->adj_order[first].z >> 16))) {
+        while (desc.size() % aw) desc.push_back(make_int4(-1, 0, ctx->adj_order[first].z & ~0xffff, 0));
+        first = q;
+      }
+      desc.push_back(e);
+    }
+    while (desc.size() % aw) desc.push_back(make_int4(-1, 0, desc.back().z & ~0xffff, 0));
+    a.ngroups = (int)(desc.size() / aw);
+    a.desc = dupload(ctx, desc.data(), desc.size());
+    R.order = dalloc<unsigned short>(ctx, R.nfun * Np);
+    R.off = dalloc<unsigned short>(ctx, (size_t)R.nseg * (R.nb + R.nfun));
+    R.item = dalloc<unsigned short>(ctx, (size_t)R.nseg * (R.nb + 1));
+    R.slot_atom = dalloc<int>(ctx, Np);
+    a.warps = sh.warps;
+    a.ctas = std::max(1, std::min(sh.per_sm * ctx->nsm, (a.ngroups + a.warps - 1) / a.warps));
+    a.rctas = std::max(1, std::min(R.nseg, 4 * ctx->nsm));
+    ra.len = sh.part;
+    ra.nang = sh.nang;
+    // partials and sums, in the buffer of k_adj's FP64 tables where they fit
+    const size_t np = (size_t)a.ctas * ra.len, nr = (size_t)a.rctas * 4 * R.nb;
+    const size_t need = C * (np + nr + ra.len + 4 * (size_t)R.nb);
+    double *buf = need <= ctx->wglob_len ? ctx->d_wglob : dalloc<double>(ctx, need);
+    a.part = buf;
+    a.rpart = buf + C * np;
+    ra.sum = a.rpart + C * nr;
+    ra.rsum = ra.sum + C * ra.len;
+    ck(rows_sort(ctx->db, ctx->pot, R, ctx->stream), "k_rows_sort launch");
+    ck(cudaStreamSynchronize(ctx->stream), "k_rows_sort");
+  } catch (const Failure &f) {
+    if (f.status != MZ_ERR_NOMEM) throw;
+    cudaGetLastError();  // the failed allocation's code
+    while (ctx->allocs.size() > mark) {
+      cudaFree(ctx->allocs.back());
+      ctx->allocs.pop_back();
+    }
+    ra.failed = true;
+    return false;
+  }
+  ra.ready = true;
+  return true;
+}
+
+void enqueue_rows_adj(mz_ctx *ctx, int n, double *d_grad) {
+  auto &ra = ctx->radj;
+  RowsAdjoint a = ra.args;
+  a.ncand = n;
+  a.geom = ctx->d_geom;
+  a.tabs = ctx->d_tabs;
+  a.ptabs = ctx->d_ptabs;
+  a.aout = ctx->d_aout;
+  a.aux = a.meam ? ctx->d_aux : nullptr;
+  a.lam = ctx->d_lam;
+  a.seeds = ctx->d_seeds;
+  a.W1 = ctx->d_V;
+  a.stream = ctx->stream;
+  {
+    Bracket b(ctx, MZ_K_ADJ);
+    ck(rows_adjoint(a), "k_rows_adj launch");
+  }
+  {
+    Bracket b(ctx, MZ_K_RADIAL);
+    ck(rows_radial(a), "k_rows_radial launch");
+  }
+  GradSums g{};
+  g.partial[0] = a.part;
+  g.sum[0] = ra.sum;
+  g.nparts[0] = a.ctas;
+  g.len[0] = ra.len;
+  g.partial[1] = a.rpart;
+  g.sum[1] = ra.rsum;
+  g.nparts[1] = a.rctas;
+  g.len[1] = 4 * a.radial.nb;
+  launch_grad_sum(ctx, n, g);
+  Bracket b(ctx, MZ_K_GRAD_FINAL);
+  k_rows_grad_final<<<n, 256, 2 * sizeof(double) * ctx->stride, ctx->stream>>>(
+      ctx->pot, a.radial, ra.nang, ctx->d_geom, ctx->d_tabs, ra.sum, ra.rsum, ctx->d_M, ctx->d_cmap, ctx->P, d_grad);
+  ck(cudaGetLastError(), "k_rows_grad_final launch");
 }
 
 // ------------------------------------------------------- triplet moments
@@ -668,6 +808,10 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
     ck(cudaGetLastError(), "k_cells launch");
   }
   if (!grad) return;
+  if (!mixed && ctx->radj.ready) {
+    enqueue_rows_adj(ctx, n, d_grad);
+    return;
+  }
   {
     Bracket b(ctx, MZ_K_ADJ);
     const size_t sj = ctx->smem_adj[mixed ? 1 : 0];
@@ -937,6 +1081,7 @@ double trial(mz_ctx *ctx, int n, const double *d_params, int precision, bool gra
 // the adjoint's atoms per block and persistent CTAs, by timing each on the
 // caller's own candidates; MZ_TUNE=0 keeps the first variant of each.
 void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, bool grad) {
+  if (precision == MZ_FP64 && grad) rows_adj_prepare(ctx);
   mz_ctx::Tune &t = ctx->tune[precision][grad ? 1 : 0];
   if (!t.done) {
     const std::vector<int64_t> key = {ctx->device,     ctx->natoms,    ctx->npairs, ctx->ncells, ctx->pot.style,
@@ -960,7 +1105,9 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
         best.adj_nc = 2;
         best.ctas = adj_ctas_for(ctx, 0, ctx->adj2_per_sm);
       }
-      if (ctx->autotune == 1) {
+      // the FP64 row kernels have no variants to time
+      const bool fixed = precision == MZ_FP64 && ctx->rows_ok && (!grad || ctx->radj.ready);
+      if (ctx->autotune == 1 && !fixed) {
         const int64_t l0 = ctx->launches;
         apply_variant(ctx, best);
         trial(ctx, n, d_params, precision, grad, MZ_K_ATOMS);  // warm-up
@@ -1196,6 +1343,12 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
       dp.s_q[m] = m < dp.nj ? pot.spline_index(m == 0 ? G_Q1 : G_Q2, 0) : 0;
     }
     dp.aux_rows = AUX_COUNT * (1 + dp.nj);
+    for (int t = 0; t < dp.npair; ++t) {
+      ctx->radial_nint[0] = std::max(ctx->radial_nint[0], geom[dp.s_phi + t].n - 1);
+      if (meam) ctx->radial_nint[2] = std::max(ctx->radial_nint[2], geom[dp.s_f + t].n - 1);
+    }
+    for (int t = 0; t < pot.ntypes && !dp.pair; ++t)
+      ctx->radial_nint[1] = std::max(ctx->radial_nint[1], geom[dp.s_rho + t].n - 1);
     dp.ang_cover = 1;
     if (meam) {
       dp.ang_p0 = geom[dp.s_g].poff / 4;
@@ -1310,6 +1463,12 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
       std::stable_sort(order.begin(), order.end(),
                        [&](int a, int b) { return db.atom_type[a] < db.atom_type[b]; });
       d.adj_atoms = dupload(ctx, order.data(), order.size());
+      ctx->adj_order.resize(N);
+      for (int q = 0; q < N; ++q) {
+        const int i = order[q];
+        ctx->adj_order[q] = make_int4(i, (int)db.pair_off[i], (int)(db.pair_off[i + 1] - db.pair_off[i]) | db.atom_type[i] << 16,
+                                      db.atom_cell[i]);
+      }
       for (int v = 0; v < mz_ctx::NCAPS; ++v) {
         const int cap = TUNE_CAPS[v], acap = std::max(1, cap / 4);
         std::vector<int> b0(1, 0);
@@ -1586,7 +1745,8 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     ctx->d_seeds = dalloc<double>(ctx, C * CS_COUNT * db.ncells);
     const size_t nparts = std::max<size_t>(ctx->adj_ctas_max, (ctx->nadjblk[0] + d.adj_group - 1) / d.adj_group);
     ctx->d_partial = dalloc<double>(ctx, C * nparts * stride);
-    ctx->d_wglob = dalloc<double>(ctx, C * (size_t)ctx->adj_ctas_max * ADJ_WARPS * stride);
+    ctx->wglob_len = C * (size_t)ctx->adj_ctas_max * ADJ_WARPS * stride;
+    ctx->d_wglob = dalloc<double>(ctx, ctx->wglob_len);
     ctx->d_grad = dalloc<double>(ctx, C * ctx->P);
     ctx->d_gsum = dalloc<double>(ctx, C * stride);
     ctx->d_count = dalloc<int>(ctx, C);
@@ -1736,7 +1896,8 @@ mz_status mz_gram_device(mz_ctx *ctx, int na, const double *d_a, int64_t lda, in
 const char *mz_kernel_name(int k) {
   static const char *names[MZ_NKERNELS] = {"k_prep",   "k_atoms",      "k_force",   "k_cells",  "k_final",
                                            "k_adj",    "k_grad_final", "k_fm_coef", "k_fm_fwd", "k_fm_epi",
-                                           "k_fm_pre", "k_fm_adj",     "k_fm_grad",    "k_grad_sum"};
+                                           "k_fm_pre", "k_fm_adj",     "k_fm_grad",    "k_grad_sum",
+                                           "k_rows_radial"};
   return (k >= 0 && k < MZ_NKERNELS) ? names[k] : "?";
 }
 
