@@ -58,6 +58,75 @@
 
 using namespace mzb;
 
+// Pinned host memory is slow to get (a millisecond per megabyte), so buffers
+// of destroyed contexts serve the next ones: at most PINNED_KEEP bytes lie
+// idle, and all idle ones are freed with the process's last context.
+struct Pinned {
+  unsigned char *p = nullptr;
+  size_t bytes = 0;
+};
+class PinnedPool {
+  static constexpr size_t PINNED_KEEP = 16u << 20;
+  std::mutex mu;
+  std::vector<Pinned> idle;
+  size_t kept = 0;
+  int contexts = 0;
+
+ public:
+  void enter() {
+    std::lock_guard<std::mutex> lk(mu);
+    ++contexts;
+  }
+  void leave() {
+    std::lock_guard<std::mutex> lk(mu);
+    if (--contexts > 0) return;
+    for (auto &b : idle) cudaFreeHost(b.p);
+    idle.clear();
+    kept = 0;
+  }
+  // a buffer of at least `bytes` (an idle one of up to four times as much), or null
+  Pinned get(size_t bytes) {
+    bytes = (bytes + 0xffff) & ~size_t(0xffff);
+    {
+      std::lock_guard<std::mutex> lk(mu);
+      size_t at = idle.size();
+      for (size_t i = 0; i < idle.size(); ++i)
+        if (idle[i].bytes >= bytes && idle[i].bytes <= 4 * bytes && (at == idle.size() || idle[i].bytes < idle[at].bytes))
+          at = i;
+      if (at < idle.size()) {
+        const Pinned b = idle[at];
+        idle.erase(idle.begin() + at);
+        kept -= b.bytes;
+        return b;
+      }
+    }
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();  // the failed allocation's code
+      return Pinned{};
+    }
+    return Pinned{static_cast<unsigned char *>(p), bytes};
+  }
+  void put(Pinned &b) {
+    if (!b.p) return;
+    {
+      std::lock_guard<std::mutex> lk(mu);
+      if (kept + b.bytes <= PINNED_KEEP) {
+        idle.push_back(b);
+        kept += b.bytes;
+        b = Pinned{};
+        return;
+      }
+    }
+    cudaFreeHost(b.p);
+    b = Pinned{};
+  }
+};
+PinnedPool &pinned_pool() {
+  static PinnedPool *pool = new PinnedPool;  // never destroyed: contexts may outlive static objects
+  return *pool;
+}
+
 struct mz_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -155,6 +224,17 @@ struct mz_ctx {
   int fm8a_mode = 1;  // MZ_FM8ADJ=0 keeps the adjoint contraction on the CUDA cores
   int smem_optin = 0;  // largest dynamic shared memory a block may opt into
   bool fm_on = false;  // the moment path in force for mixed launches
+  // Host-buffer calls: coefficients, objectives, gradients and the failure flag
+  // in pinned host memory that the kernels read and write themselves (a few
+  // kilobytes over PCIe inside the launch sequence instead of copies around
+  // it), and a pinned area that larger outputs pass through.  Taken at the
+  // first such call; without it the calls copy from and to the
+  // caller's pageable memory.
+  Pinned io, io_stage;
+  bool io_tried = false, counted = false;
+  double *c_params = nullptr, *c_obj = nullptr, *c_grad = nullptr;  // what the host calls' launches use
+  int *c_flag = nullptr;
+  bool waits = false;  // kernels that can set the failure flag were launched since it was last read
   double *d_gram = nullptr;  // partial sums of mz_gram_device, grown on demand
   size_t gram_cap = 0;       // doubles
   struct Mark {
@@ -226,12 +306,18 @@ void release(mz_ctx *ctx) {
   if (ctx->d_gram) cudaFree(ctx->d_gram);
   ctx->d_gram = nullptr;
   ctx->gram_cap = 0;
+  pinned_pool().put(ctx->io);
+  pinned_pool().put(ctx->io_stage);
+  if (ctx->counted) pinned_pool().leave();
+  ctx->counted = false;
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   ctx->stream = nullptr;
 }
 
 // A kernel that gave up on a bounded wait sets the context's flag.
 void check_device_flag(mz_ctx *ctx) {
+  if (!ctx->waits) return;
+  ctx->waits = false;
   int e = 0;
   ck(cudaMemcpy(&e, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost), "flag D2H");
   if (e) {
@@ -672,6 +758,7 @@ void enqueue_fm(mz_ctx *ctx, int n, double *d_obj, double *d_errvec, double *d_f
     Bracket b(ctx, MZ_K_FM_FWD);
     const int ntile8 = (int)(fp.Q / FM8_TM);
     k_fm_gemm_fwd8<<<dim3(std::min(ntile8, ctx->nsm), G), FM8_THREADS, fm8_smem(fp.nt), st>>>(fp, ctx->d_err);
+    ctx->waits = true;
     ck(cudaGetLastError(), "k_fm_gemm_fwd8 launch");
   } else {
     {
@@ -749,7 +836,8 @@ void enqueue_fm(mz_ctx *ctx, int n, double *d_obj, double *d_errvec, double *d_f
 }
 
 // Enqueue the objective (and, with d_grad, its gradient) of n candidates
-// whose coefficient vectors are already on the device.
+// whose coefficient vectors the device can read.  Without d_obj (FP64) only
+// the per-atom densities.
 void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *d_obj, double *d_errvec,
              double *d_forces, double *d_energy, double *d_stress, double *d_grad) {
   cudaStream_t st = ctx->stream;
@@ -775,6 +863,7 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
                     ctx->d_ptabs, ctx->d_V,   ctx->d_aout,  grad && meam ? ctx->d_aux : nullptr, st};
       ck(rows_forward(a), "k_rows launch");
     } else if (meam && mixed && ctx->tc_ok) {
+      ctx->waits = true;
       dim3 gt(std::min(ctx->nsm, ctx->natoms), (n + TC_CANDS - 1) / TC_CANDS);
       const size_t st_bytes = (size_t)ctx->tc.smem_bytes;
       if (grad)
@@ -794,6 +883,7 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
     }
     ck(cudaGetLastError(), "k_atoms launch");
   }
+  if (!d_obj) return;
   {
     Bracket b(ctx, MZ_K_GATHER);
     k_force<<<dim3((unsigned)(((int64_t)ctx->natoms * FORCE_LANES + 255) / 256), n), 256, 0, st>>>(
@@ -1182,15 +1272,52 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
   apply_variant(ctx, t);
 }
 
+// Kernels with bounded waits, which can set the context's failure flag, run
+// in this precision: the tensor-core forward and the moment path's contractions.
+bool may_give_up(const mz_ctx *ctx, int precision) {
+  return precision == MZ_MIXED && (ctx->tc_ok || (ctx->fm_on && ctx->fm.ready && ctx->fm.tc8));
+}
+
+// The pinned buffers of the host calls.
+constexpr size_t IO_MAX = 16u << 20;     // coefficients, objectives and gradients of one launch
+constexpr size_t IO_STAGE = 4u << 20;    // other outputs of one launch
+void host_io(mz_ctx *ctx) {
+  if (ctx->io_tried) return;
+  ctx->io_tried = true;
+  ctx->c_params = ctx->d_params;
+  ctx->c_obj = ctx->d_obj;
+  ctx->c_grad = ctx->d_grad;
+  const size_t C = ctx->cand_cap, P = ctx->P, bytes = sizeof(double) * C * (2 * P + 1) + sizeof(double);
+  if (bytes > IO_MAX) return;
+  ctx->io = pinned_pool().get(bytes);
+  if (!ctx->io.p) return;
+  ctx->c_params = reinterpret_cast<double *>(ctx->io.p);
+  ctx->c_obj = ctx->c_params + C * P;
+  ctx->c_grad = ctx->c_obj + C;
+  ctx->c_flag = reinterpret_cast<int *>(ctx->c_grad + C * P);
+  *ctx->c_flag = 0;
+}
+// The staging area, where the outputs fit it (null: copy straight to the caller).
+unsigned char *host_stage(mz_ctx *ctx, size_t bytes) {
+  if (!ctx->io.p || bytes == 0 || bytes > IO_STAGE) return nullptr;
+  if (ctx->io_stage.bytes < bytes) {
+    pinned_pool().put(ctx->io_stage);
+    ctx->io_stage = pinned_pool().get(bytes);
+  }
+  return ctx->io_stage.p;
+}
+
 // The kernels of one objective call on the context's own buffers: captured
 // into a CUDA graph the first time a shape is seen, replayed afterwards (not
 // while profiling, whose per-kernel events are recorded around launches).
 constexpr size_t MAX_GRAPHS = 32;
 void launch_objective(mz_ctx *ctx, int n, int precision, bool ev, bool fo, bool en, bool st, bool gr) {
-  tune_variant(ctx, n, ctx->d_params, precision, gr);
+  tune_variant(ctx, n, ctx->c_params, precision, gr);
   auto go = [&] {
-    enqueue(ctx, n, ctx->d_params, precision, ctx->d_obj, ev ? ctx->d_errvec : nullptr, fo ? ctx->d_forces : nullptr,
-            en ? ctx->d_energy : nullptr, st ? ctx->d_stress : nullptr, gr ? ctx->d_grad : nullptr);
+    enqueue(ctx, n, ctx->c_params, precision, ctx->c_obj, ev ? ctx->d_errvec : nullptr, fo ? ctx->d_forces : nullptr,
+            en ? ctx->d_energy : nullptr, st ? ctx->d_stress : nullptr, gr ? ctx->c_grad : nullptr);
+    if (ctx->c_flag && may_give_up(ctx, precision))
+      ck(cudaMemcpyAsync(ctx->c_flag, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "flag D2H");
   };
   if (!ctx->use_graphs || ctx->profiling) {
     go();
@@ -1233,37 +1360,53 @@ void run_host(mz_ctx *ctx, int ncand, const double *params, int precision, doubl
   if (precision != MZ_FP64 && precision != MZ_MIXED) throw Failure{MZ_ERR_ARG, "unknown precision"};
   if (grad) check_adjoint(ctx, precision);
   ck(cudaSetDevice(ctx->device), "cudaSetDevice");
-  const int P = ctx->P, E = ctx->esize, N = ctx->natoms, NC = ctx->ncells;
+  const size_t P = ctx->P, E = ctx->esize, N = ctx->natoms, NC = ctx->ncells;
+  host_io(ctx);
   for (int c0 = 0; c0 < ncand; c0 += ctx->cand_cap) {
     const int n = std::min(ctx->cand_cap, ncand - c0);
-    ck(cudaMemcpyAsync(ctx->d_params, params + (size_t)c0 * P, sizeof(double) * n * P, cudaMemcpyHostToDevice,
-                       ctx->stream),
-       "params H2D");
+    const double *px = params + (size_t)c0 * P;
+    if (ctx->io.p) std::memcpy(ctx->c_params, px, sizeof(double) * n * P);
+    else
+      ck(cudaMemcpyAsync(ctx->d_params, px, sizeof(double) * n * P, cudaMemcpyHostToDevice, ctx->stream), "params H2D");
     launch_objective(ctx, n, precision, errvec != nullptr, forces != nullptr, energy != nullptr, stress != nullptr,
                      grad != nullptr);
-    ck(cudaMemcpyAsync(obj + c0, ctx->d_obj, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream), "obj D2H");
-    if (grad)
-      ck(cudaMemcpyAsync(grad + (size_t)c0 * P, ctx->d_grad, sizeof(double) * n * P, cudaMemcpyDeviceToHost,
-                         ctx->stream),
-         "grad D2H");
-    if (errvec)
-      ck(cudaMemcpyAsync(errvec + (size_t)c0 * E, ctx->d_errvec, sizeof(double) * n * E, cudaMemcpyDeviceToHost,
-                         ctx->stream),
-         "errvec D2H");
-    if (forces)
-      ck(cudaMemcpyAsync(forces + (size_t)c0 * 3 * N, ctx->d_forces, sizeof(double) * n * 3 * N,
-                         cudaMemcpyDeviceToHost, ctx->stream),
-         "forces D2H");
-    if (energy)
-      ck(cudaMemcpyAsync(energy + (size_t)c0 * NC, ctx->d_energy, sizeof(double) * n * NC, cudaMemcpyDeviceToHost,
-                         ctx->stream),
-         "energy D2H");
-    if (stress)
-      ck(cudaMemcpyAsync(stress + (size_t)c0 * 6 * NC, ctx->d_stress, sizeof(double) * n * 6 * NC,
-                         cudaMemcpyDeviceToHost, ctx->stream),
-         "stress D2H");
+    struct Out {
+      double *host;
+      const double *dev;
+      size_t count;
+    };
+    Out outs[6] = {{errvec ? errvec + c0 * E : nullptr, ctx->d_errvec, n * E},
+                   {forces ? forces + c0 * 3 * N : nullptr, ctx->d_forces, n * 3 * N},
+                   {energy ? energy + c0 * NC : nullptr, ctx->d_energy, n * NC},
+                   {stress ? stress + c0 * 6 * NC : nullptr, ctx->d_stress, n * 6 * NC},
+                   {ctx->io.p ? nullptr : obj + c0, ctx->d_obj, (size_t)n},
+                   {ctx->io.p || !grad ? nullptr : grad + c0 * P, ctx->d_grad, n * P}};
+    size_t bytes = 0;
+    for (auto &o : outs) bytes += o.host ? sizeof(double) * o.count : 0;
+    unsigned char *stage = host_stage(ctx, bytes), *at = stage;
+    for (auto &o : outs) {
+      if (!o.host) continue;
+      const size_t b = sizeof(double) * o.count;
+      ck(cudaMemcpyAsync(stage ? (void *)at : (void *)o.host, o.dev, b, cudaMemcpyDeviceToHost, ctx->stream),
+         "output D2H");
+      at += stage ? b : 0;
+    }
     ck(cudaStreamSynchronize(ctx->stream), "objective");
-    check_device_flag(ctx);
+    if (ctx->io.p) {
+      std::memcpy(obj + c0, ctx->c_obj, sizeof(double) * n);
+      if (grad) std::memcpy(grad + c0 * P, ctx->c_grad, sizeof(double) * n * P);
+    }
+    at = stage;
+    for (auto &o : outs)
+      if (o.host && stage) {
+        std::memcpy(o.host, at, sizeof(double) * o.count);
+        at += sizeof(double) * o.count;
+      }
+    if (may_give_up(ctx, precision) && (!ctx->c_flag || *ctx->c_flag)) {
+      if (ctx->c_flag) *ctx->c_flag = 0;
+      ctx->waits = true;  // a replayed graph does not set it
+      check_device_flag(ctx);
+    }
   }
 }
 
@@ -1294,6 +1437,8 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
           }
     ctx = new mz_ctx;
     ctx->device = set->device;
+    pinned_pool().enter();
+    ctx->counted = true;
     ck(cudaSetDevice(ctx->device), "cudaSetDevice");
     ck(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     ctx->natoms = db.natoms;
@@ -1817,14 +1962,20 @@ mz_status mz_densities(mz_ctx *ctx, const double *params, double *dens) {
     if (ctx->pot.pair)  // PotPair has no compute_densities (pot_pair.h:25-42)
       throw Failure{MZ_ERR_UNSUPPORTED, "pair/spline has no embedding densities"};
     ck(cudaSetDevice(ctx->device), "cudaSetDevice");
-    ck(cudaMemcpyAsync(ctx->d_params, params, sizeof(double) * ctx->P, cudaMemcpyHostToDevice, ctx->stream),
-       "params H2D");
-    tune_variant(ctx, 1, ctx->d_params, MZ_FP64, false);
-    enqueue(ctx, 1, ctx->d_params, MZ_FP64, ctx->d_obj, nullptr, nullptr, nullptr, nullptr, nullptr);
-    ck(cudaMemcpyAsync(dens, ctx->d_aout + (size_t)AO_RHO * ctx->natoms, sizeof(double) * ctx->natoms,
+    host_io(ctx);
+    if (ctx->io.p) std::memcpy(ctx->c_params, params, sizeof(double) * ctx->P);
+    else
+      ck(cudaMemcpyAsync(ctx->d_params, params, sizeof(double) * ctx->P, cudaMemcpyHostToDevice, ctx->stream),
+         "params H2D");
+    tune_variant(ctx, 1, ctx->c_params, MZ_FP64, false);
+    enqueue(ctx, 1, ctx->c_params, MZ_FP64, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);  // to the densities
+    const size_t bytes = sizeof(double) * ctx->natoms;
+    unsigned char *stage = host_stage(ctx, bytes);
+    ck(cudaMemcpyAsync(stage ? (void *)stage : (void *)dens, ctx->d_aout + (size_t)AO_RHO * ctx->natoms, bytes,
                        cudaMemcpyDeviceToHost, ctx->stream),
        "dens D2H");
     ck(cudaStreamSynchronize(ctx->stream), "densities");
+    if (stage) std::memcpy(dens, stage, bytes);
   });
 }
 
