@@ -237,6 +237,7 @@ struct mz_ctx {
   bool waits = false;  // kernels that can set the failure flag were launched since it was last read
   double *d_gram = nullptr;  // partial sums of mz_gram_device, grown on demand
   size_t gram_cap = 0;       // doubles
+  bool gram_ready[2] = {false, false};  // shared memory of k_gram_tile set (narrow, wide copies)
   struct Mark {
     int kernel;
     cudaEvent_t start, stop;
@@ -2011,8 +2012,10 @@ mz_status mz_gram_device(mz_ctx *ctx, int na, const double *d_a, int64_t lda, in
     const int64_t units = (n + unit - 1) / unit;
     const int Ti = (na + GRAM_T - 1) / GRAM_T, Tj = (nb + GRAM_T - 1) / GRAM_T;
     const int ntiles = vec ? 1 : (g.sym ? Tj * (Tj + 1) / 2 : Ti * Tj);
-    // about four CTAs per SM over all tiles and k ranges
-    const int64_t want = std::max<int64_t>(1, (4 * (int64_t)ctx->nsm + ntiles - 1) / ntiles);
+    // the vector form: four CTAs per SM over the k ranges; the tiles: one (its
+    // eight warps keep the FP64 pipe busy, and fewer ranges leave fewer partials)
+    const int64_t per_sm = vec ? 4 : 1;
+    const int64_t want = std::max<int64_t>(1, per_sm * (int64_t)ctx->nsm / ntiles);
     int64_t S = std::min(units, want);
     const int64_t per = (units + S - 1) / S;
     S = (units + per - 1) / per;  // no empty range
@@ -2034,11 +2037,18 @@ mz_status mz_gram_device(mz_ctx *ctx, int na, const double *d_a, int64_t lda, in
     g.partial = ctx->d_gram;
     if (vec)
       k_gram_vec<<<(unsigned)S, 256, 0, ctx->stream>>>(g);
-    else
-      k_gram_tile<<<dim3((unsigned)ntiles, (unsigned)S), 256, 0, ctx->stream>>>(g);
+    else {
+      const size_t sm = gram_smem(g.sym && ntiles == 1);
+      // 16-byte copies where every row starts on one (g.kper is a multiple of 32)
+      const bool wide = ((uintptr_t)d_a | (uintptr_t)d_b) % 16 == 0 && lda % 2 == 0 && ldb % 2 == 0;
+      auto k = wide ? k_gram_tile<true> : k_gram_tile<false>;
+      if (!ctx->gram_ready[wide]) smem_attr(k, gram_smem(false));
+      ctx->gram_ready[wide] = true;
+      k<<<dim3((unsigned)ntiles, (unsigned)S), 256, sm, ctx->stream>>>(g);
+    }
     ck(cudaGetLastError(), "k_gram");
     const int outs = na * nb;
-    k_gram_sum<<<(outs + 255) / 256, 256, 0, ctx->stream>>>(g);
+    k_gram_sum<<<(outs + 31) / 32, 1024, 0, ctx->stream>>>(g);
     ck(cudaGetLastError(), "k_gram_sum");
     ctx->launches += 2;
   });
