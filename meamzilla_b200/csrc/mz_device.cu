@@ -645,7 +645,7 @@ bool fm_prepare(mz_ctx *ctx) {
   size_t extra = sizeof(float) * 3 * (size_t)fp.Dpad * Q + sizeof(double) * 8 * Q + sizeof(float) * G * fp.nt * fp.Dpad * CG +
                  sizeof(double) * C * ns * FM_MAXB + sizeof(float) * G * ns * FM_MAXB * CG +
                  sizeof(double) * G * CG *
-                     ((size_t)fp.nctas_adj * fp.nt * fp.Dpad + (size_t)fp.nctas_pre * (ns * FM_MAXB + stride));
+                     ((size_t)(fp.nctas_adj + 1) * fp.nt * fp.Dpad + (size_t)(fp.nctas_pre + 1) * (ns * FM_MAXB + stride));
   for (auto &x : need)
     if (x.need_bytes > x.have_bytes) extra += x.need_bytes;
   size_t freeb = 0, totalb = 0;
@@ -698,6 +698,7 @@ bool fm_prepare(mz_ctx *ctx) {
   fp.Kbar = dalloc<double>(ctx, G * fp.nctas_adj * fp.nt * fp.Dpad * CG);
   fp.Pbar = dalloc<double>(ctx, G * fp.nctas_pre * ns * FM_MAXB * CG);
   fp.Tbar = dalloc<double>(ctx, G * fp.nctas_pre * CG * stride);
+  fp.sums = dalloc<double>(ctx, G * CG * (fp.nt * fp.Dpad + ns * FM_MAXB + stride));
   if (X) ck(cudaMemsetAsync(X, 0, sizeof(float) * 3 * (size_t)fp.Dpad * Q, ctx->stream), "memset");
   ck(cudaMemsetAsync(E, 0, sizeof(double) * 8 * Q, ctx->stream), "memset");
   ck(cudaMemsetAsync(coef64, 0, sizeof(double) * C * ns * FM_MAXB, ctx->stream), "memset");
@@ -753,7 +754,7 @@ void enqueue_fm(mz_ctx *ctx, int n, double *d_obj, double *d_errvec, double *d_f
   if (ctx->fm.tc8) {  // the forward contraction in integers on the tensor cores
     {
       Bracket b(ctx, MZ_K_FM_COEF);
-      k_fm_kmat8<<<dim3(fp.nt, G), 256, 0, st>>>(n, ctx->pot, fp, fp.coef64, fp.K8, fp.ke);
+      k_fm_kmat8<<<dim3(fp.nt, G, FM8_NC / FM8_KC), 32 * FM8_KC, 0, st>>>(n, ctx->pot, fp, fp.coef64, fp.K8, fp.ke);
       ck(cudaGetLastError(), "k_fm_kmat8 launch");
     }
     Bracket b(ctx, MZ_K_FM_FWD);
@@ -796,8 +797,7 @@ void enqueue_fm(mz_ctx *ctx, int n, double *d_obj, double *d_errvec, double *d_f
   }
   {
     Bracket b(ctx, MZ_K_CELLS);
-    const unsigned cblocks = (unsigned)(((int64_t)NC * CG + 255) / 256);
-    k_fm_cells<<<dim3(cblocks, G), 256, 0, st>>>(ctx->db, ctx->pot, fp, n, ctx->d_cellobj, d_errvec, ctx->esize,
+    k_fm_cells<<<dim3(NC, G), CG * FM_CSL, 0, st>>>(ctx->db, ctx->pot, fp, n, ctx->d_cellobj, d_errvec, ctx->esize,
                                                  d_energy, d_stress, grad ? 1 : 0);
     ck(cudaGetLastError(), "k_fm_cells launch");
   }
@@ -829,8 +829,11 @@ void enqueue_fm(mz_ctx *ctx, int n, double *d_obj, double *d_errvec, double *d_f
   }
   {
     Bracket b(ctx, MZ_K_FM_GRAD);
-    const size_t sm = sizeof(double) * ((size_t)ns * FM_MAXB + ctx->stride + (size_t)fp.nt * fp.Dpad);
-    k_fm_grad<<<n, 256, sm, st>>>(ctx->pot, ctx->d_geom, fp, fp.coef64, ctx->d_partial);
+    const int sums = fp.nt * fp.Dpad + ns * FM_MAXB + ctx->stride;
+    k_fm_sum<<<dim3((sums * CG + 255) / 256, G), 256, 0, st>>>(ctx->pot, fp, fp.sums);
+    ck(cudaGetLastError(), "k_fm_sum launch");
+    ctx->launches += 1;
+    k_fm_grad<<<n, 256, sizeof(double) * sums, st>>>(ctx->pot, ctx->d_geom, fp, fp.coef64, fp.sums, ctx->d_partial);
     ck(cudaGetLastError(), "k_fm_grad launch");
   }
   launch_grad_final(ctx, n, 1, d_grad);

@@ -31,7 +31,7 @@
 //   E     [Q][8]                     e1, e2 of the slot (FP64)
 //   Y     [ngroups][Q][3][CG]        G, Y1, Y2 (FP32)
 //   Yb    [ngroups][Q][3][CG]        dL/dG, dL/dY1, dL/dY2 (FP32)
-//   V     [ngroups][Np][CG][3]       reaction vectors (FP64), global slot order
+//   V     [ngroups][Np][3][CG]       reaction vectors (FP64), global slot order
 //   aoutF [ngroups][N][AO_COUNT][CG] per-atom outputs (FP64)
 // with candidates in groups of CG (the launch's candidates rounded up to a
 // power of two from 8 to 64).
@@ -80,7 +80,8 @@ struct FmPlan {
   double *seedF;           // [ngroups][NC][CS_COUNT][CG]
   double *Kbar;            // [ngroups][nctas_adj][nt][Dpad][CG]  FP64 partials of the adjoint contraction
   double *Pbar;            // [ngroups][nctas_pre][nsplines][FM_MAXB][CG]  pair-function B-spline gradients
-  double *Tbar;            // [ngroups][nctas_pre][CG][stride]  embedding table gradients
+  double *Tbar;            // [ngroups][nctas_pre][stride][CG]  embedding table gradients
+  double *sums;            // [ngroups][nt Dpad + nsplines FM_MAXB + stride][CG] their sums (k_fm_sum)
   int nctas_adj, nctas_pre;
   // the integer contraction (mz_fm8.cuh), when built
   const signed char *X8;   // [Q / 128][3][2][3][16 KB]
@@ -711,7 +712,7 @@ __global__ void __launch_bounds__(256) k_fm_epi(DevDb db, DevPot pot, const Spli
   const int c = gy * CG + cl;
   const bool live = c < ncand;
   const double *tc = tabs + (size_t)(live ? c : 0) * pot.tab_stride;
-  double *__restrict__ Vg = fp.V + (size_t)gy * db.npairs * CG * 3 + cl * 3;
+  double *__restrict__ Vg = fp.V + (size_t)gy * db.npairs * CG * 3 + cl;
   for (int blk = blockIdx.x; blk < fp.nblk; blk += gridDim.x) {
     int na, ti;
     const int nslot = fm_stage_block<double>(db, pot, sg, fp, st, blk, gy, ncand, na, ti);
@@ -778,8 +779,8 @@ __global__ void __launch_bounds__(256) k_fm_epi(DevDb db, DevPot pot, const Spli
         const double Vz = dz * A + B * (e[2] * Y1 + e[5] * Y2);
         double *Vd = Vg + (size_t)gs * CG * 3;
         Vd[0] = Vx;
-        Vd[1] = Vy;
-        Vd[2] = Vz;
+        Vd[CG] = Vy;
+        Vd[2 * CG] = Vz;
         F[0] += Vx;
         F[1] += Vy;
         F[2] += Vz;
@@ -818,13 +819,14 @@ __global__ void k_fm_gather(DevDb db, FmPlan fp, int ncand, double *__restrict__
   const int i = (int)(idx / CG), cl = (int)(idx % CG), c = gy * CG + cl;
   if (c >= ncand) return;
   double *ao = fp.aoutF + ((size_t)gy * N + i) * AO_COUNT * CG + cl;
-  const double *Vg = fp.V + (size_t)gy * db.npairs * CG * 3 + cl * 3;
+  const double *Vg = fp.V + (size_t)gy * db.npairs * CG * 3 + cl;
   double fx = ao[AO_AX * CG], fy = ao[AO_AY * CG], fz = ao[AO_AZ * CG];
+#pragma unroll 4
   for (int q = db.in_off[i]; q < db.in_off[i + 1]; ++q) {
     const double *v = Vg + (size_t)db.in_slot[q] * CG * 3;
     fx -= v[0];
-    fy -= v[1];
-    fz -= v[2];
+    fy -= v[CG];
+    fz -= v[2 * CG];
   }
   const int cell = db.atom_cell[i];
   const double w = db.cell_w[cell];
@@ -855,30 +857,50 @@ __global__ void k_fm_gather(DevDb db, FmPlan fp, int ncand, double *__restrict__
 
 // -------------------------------------------------------------- k_fm_cells
 
-// Potential::accumulate_error per cell (potential.cpp:450-485), thread =
-// (cell, candidate); with want_seeds also the adjoint seeds dF/dE_atom,
-// dF/dS_cell / volume and dF/dpen.
-__global__ void k_fm_cells(DevDb db, DevPot pot, FmPlan fp, int ncand, double *__restrict__ cellobj,
-                           double *__restrict__ errvec, int esize, double *__restrict__ energy,
-                           double *__restrict__ stress, int want_seeds) {
+// Potential::accumulate_error per cell (potential.cpp:450-485), a CTA per
+// cell and group: the lanes are candidates, the FM_CSL slices of the CTA take
+// every FM_CSL-th atom each, and the slices' sums are added in order; with
+// want_seeds also the adjoint seeds dF/dE_atom, dF/dS_cell / volume and dF/dpen.
+// (A thread per cell and candidate walked up to 1024 atoms: 1230 us for 400
+// cells and 64 candidates, this 85.)
+constexpr int FM_CSL = 8;
+
+__global__ void __launch_bounds__(64 * FM_CSL)
+    k_fm_cells(DevDb db, DevPot pot, FmPlan fp, int ncand, double *__restrict__ cellobj,
+               double *__restrict__ errvec, int esize, double *__restrict__ energy,
+               double *__restrict__ stress, int want_seeds) {
+  __shared__ double part[FM_CSL][9][64];
   const int CG = fp.CG, gy = blockIdx.y;
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int NC = db.ncells, N = db.natoms;
-  if (idx >= (int64_t)NC * CG) return;
-  const int cell = (int)(idx / CG), cl = (int)(idx % CG), c = gy * CG + cl;
-  if (c >= ncand) return;
+  const int cell = blockIdx.x, cl = threadIdx.x % CG, sl = threadIdx.x / CG, c = gy * CG + cl;
   const int a0 = db.cell_atom0[cell], a1 = db.cell_atom0[cell + 1];
   double v[9];
 #pragma unroll
   for (int q = 0; q < 9; ++q) v[q] = 0.0;
-  for (int a = a0; a < a1; ++a) {
-    const double *ao = fp.aoutF + ((size_t)gy * N + a) * AO_COUNT * CG + cl;
-    v[0] += ao[AO_E * CG];
+  constexpr int U = 4;  // atoms whose loads are in flight together
+  constexpr int row[9] = {AO_E, AO_S0, AO_S0 + 1, AO_S0 + 2, AO_S0 + 3, AO_S0 + 4, AO_S0 + 5, AO_PEN, AO_FSQ};
+  const double *base = fp.aoutF + (size_t)gy * N * AO_COUNT * CG + cl;
+  for (int a = a0 + sl; a < a1; a += U * FM_CSL) {
+    double x[U][9];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) v[1 + q] += ao[(AO_S0 + q) * CG];
-    v[7] += ao[AO_PEN * CG];
-    v[8] += ao[AO_FSQ * CG];
+    for (int u = 0; u < U; ++u) {
+      const double *ao = base + (size_t)min(a + u * FM_CSL, a1 - 1) * AO_COUNT * CG;
+#pragma unroll
+      for (int q = 0; q < 9; ++q) x[u][q] = __ldg(ao + row[q] * CG);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (a + u * FM_CSL < a1)
+#pragma unroll
+        for (int q = 0; q < 9; ++q) v[q] += x[u][q];
   }
+#pragma unroll
+  for (int q = 0; q < 9; ++q) part[sl][q][cl] = v[q];
+  __syncthreads();
+  if (sl > 0 || c >= ncand) return;
+  for (int s = 1; s < FM_CSL; ++s)
+#pragma unroll
+    for (int q = 0; q < 9; ++q) v[q] += part[s][q][cl];
   const int na = a1 - a0;
   const double w = db.cell_w[cell];
   const double E = v[0] / na;
@@ -966,7 +988,7 @@ __global__ void __launch_bounds__(256, 2) k_fm_adj_pre(DevDb db, DevPot pot, con
   for (int e = tid; e < npe * CG; e += T) pacc[e] = 0.f;
   for (int e = tid; e < fp.ustride * CG; e += T) utab[e] = 0.0;
   double *Pb = fp.Pbar + ((size_t)gy * gridDim.x + blockIdx.x) * pot.nsplines * FM_MAXB * CG;
-  double *Tb = fp.Tbar + ((size_t)gy * gridDim.x + blockIdx.x) * CG * pot.tab_stride;
+  double *Tb = fp.Tbar + ((size_t)gy * gridDim.x + blockIdx.x) * CG * pot.tab_stride;  // [stride][CG]
   for (int i = tid; i < pot.nsplines * FM_MAXB * CG; i += T) Pb[i] = 0.0;
   for (int i = tid; i < CG * pot.tab_stride; i += T) Tb[i] = 0.0;
   // the CTA's sums of atom type tf into its FP64 partials
@@ -1160,8 +1182,8 @@ __global__ void __launch_bounds__(256, 2) k_fm_adj_pre(DevDb db, DevPot pot, con
   if (pacc_t >= 0) flush_pairs(pacc_t);
   // the embedding table sums into this CTA's partial
   for (int idx = tid; idx < fp.ustride * CG; idx += T) {
-    const int c2 = idx / fp.ustride, e = idx % fp.ustride;
-    Tb[(size_t)c2 * pot.tab_stride + fp.utoff + e] = utab[idx];
+    const int c2 = idx % CG, e = idx / CG;
+    Tb[(size_t)(fp.utoff + e) * CG + c2] = utab[(size_t)c2 * fp.ustride + e];
   }
 }
 
@@ -1345,78 +1367,103 @@ __global__ void __launch_bounds__(256, 1) k_fm_gemm_adj(FmPlan fp) {
 
 // -------------------------------------------------------------- k_fm_grad
 
-// Per candidate: the CTA partials summed in order; the contraction's Kbar
+// The CTAs' partials of Kbar, Pbar and Tbar added in order, a thread per sum
+// (neighbouring threads are neighbouring candidates):
+// out [ngroups][nt Dpad + ns FM_MAXB + stride][CG].  (k_fm_grad's CTA per
+// candidate read them 8 bytes every 512: 590 us with its serial tail for 64
+// candidates; the two kernels take 93.)
+__global__ void __launch_bounds__(256) k_fm_sum(DevPot pot, FmPlan fp, double *__restrict__ out) {
+  const int CG = fp.CG, gy = blockIdx.y, ns = pot.nsplines, stride = pot.tab_stride;
+  const int nk = fp.nt * fp.Dpad, np = ns * FM_MAXB, total = nk + np + stride;
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= total * CG) return;
+  const int e = idx / CG, cl = idx % CG;
+  const double *p;
+  size_t step;
+  int parts;
+  if (e < nk) {
+    step = (size_t)nk * CG;
+    parts = fp.nctas_adj;
+    p = fp.Kbar + (size_t)gy * parts * step + (size_t)e * CG + cl;
+  } else if (e < nk + np) {
+    step = (size_t)np * CG;
+    parts = fp.nctas_pre;
+    p = fp.Pbar + (size_t)gy * parts * step + (size_t)(e - nk) * CG + cl;
+  } else {
+    step = (size_t)CG * stride;
+    parts = fp.nctas_pre;
+    p = fp.Tbar + (size_t)gy * parts * step + (size_t)(e - nk - np) * CG + cl;
+  }
+  double v = 0.0;
+#pragma unroll 16
+  for (int b = 0; b < parts; ++b) v += p[b * step];
+  out[((size_t)gy * total + e) * CG + cl] = v;
+}
+
+// Per candidate, from those sums: the contraction's Kbar
 // split into its factors (dL/dc_a = sum_n Kbar w_n, dL/dw_n = sum_a Kbar c_a);
 // the B-spline coefficient gradients of phi, rho, f, g mapped to the knot
 // table (the transpose of k_fm_coef's map); the embedding table gradients
 // added.  The result is one table-gradient partial, which k_grad_final maps
 // to the coefficients.
-__global__ void k_fm_grad(DevPot pot, const SplineGeom *__restrict__ geom, FmPlan fp,
-                          const double *__restrict__ coef64, double *__restrict__ out) {
+__global__ void __launch_bounds__(256)
+    k_fm_grad(DevPot pot, const SplineGeom *__restrict__ geom, FmPlan fp, const double *__restrict__ coef64,
+              const double *__restrict__ sums, double *__restrict__ out) {
   extern __shared__ double gsm[];
   const int c = blockIdx.x, CG = fp.CG, gy = c / CG, cl = c % CG;
-  const int ns = pot.nsplines, stride = pot.tab_stride;
-  double *bgrad = gsm;                         // [ns][FM_MAXB]
+  const int ns = pot.nsplines, stride = pot.tab_stride, nk = fp.nt * fp.Dpad;
+  double *kbar = gsm;                          // [nt][Dpad]
+  double *bgrad = kbar + nk;                   // [ns][FM_MAXB]
   double *tab = bgrad + (size_t)ns * FM_MAXB;  // [stride]
-  double *kbar = tab + stride;                 // [nt][Dpad]
-  for (int i = threadIdx.x; i < ns * FM_MAXB; i += blockDim.x) {
-    const int s = i / FM_MAXB, a = i % FM_MAXB;
-    double v = 0.0;
-    for (int b = 0; b < fp.nctas_pre; ++b)
-      v += fp.Pbar[(((size_t)gy * fp.nctas_pre + b) * ns + s) * FM_MAXB * CG + (size_t)a * CG + cl];
-    bgrad[i] = v;
-  }
-  for (int e = threadIdx.x; e < stride; e += blockDim.x) {
-    double v = 0.0;
-    for (int b = 0; b < fp.nctas_pre; ++b) v += fp.Tbar[(((size_t)gy * fp.nctas_pre + b) * CG + cl) * stride + e];
-    tab[e] = v;
-  }
-  for (int i = threadIdx.x; i < fp.nt * fp.Dpad; i += blockDim.x) {
-    double v = 0.0;
-    for (int b = 0; b < fp.nctas_adj; ++b)
-      v += fp.Kbar[(((size_t)gy * fp.nctas_adj + b) * fp.nt * fp.Dpad + i) * CG + cl];
-    kbar[i] = v;
-  }
+  const int total = nk + ns * FM_MAXB + stride;
+  for (int e = threadIdx.x; e < total; e += blockDim.x) gsm[e] = sums[((size_t)gy * total + e) * CG + cl];
   __syncthreads();
   const double *cf = coef64 + (size_t)c * ns * FM_MAXB;
-  if (threadIdx.x == 0) {
-    // Kbar -> f and g coefficient gradients, in a fixed order
-    for (int s = 0; s < fp.nt; ++s) {
-      const int gs = pot.s_g + s;
+  // Kbar -> f and g coefficient gradients, a thread per coefficient
+  for (int i = threadIdx.x; i < ns * FM_MAXB; i += blockDim.x) {
+    const int sp = i / FM_MAXB, a = i % FM_MAXB;
+    double v = bgrad[i];
+    if (sp >= pot.s_f && sp < pot.s_f + pot.npair && a < fp.NA) {
+      for (int s = 0; s < fp.nt; ++s)
+        for (int o = 0; o < fp.nt; ++o) {
+          if (pot.s_f + pair_ij_index(s, o, pot.ntypes) != sp) continue;
+          const double *kb = kbar + (size_t)s * fp.Dpad + (o * fp.NA + a) * fp.NN;
+          const double *g = cf + (size_t)(pot.s_g + s) * FM_MAXB;
+          for (int nn = 0; nn < fp.NN; ++nn) v += kb[nn] * g[nn];
+        }
+    } else if (sp >= pot.s_g && sp < pot.s_g + fp.nt && a < fp.NN) {
+      const int s = sp - pot.s_g;
       for (int o = 0; o < fp.nt; ++o) {
-        const int fs = pot.s_f + pair_ij_index(s, o, pot.ntypes);
-        for (int a = 0; a < fp.NA; ++a)
-          for (int nn = 0; nn < fp.NN; ++nn) {
-            const double kb = kbar[(size_t)s * fp.Dpad + (o * fp.NA + a) * fp.NN + nn];
-            bgrad[(size_t)fs * FM_MAXB + a] += kb * cf[(size_t)gs * FM_MAXB + nn];
-            bgrad[(size_t)gs * FM_MAXB + nn] += kb * cf[(size_t)fs * FM_MAXB + a];
-          }
+        const double *f = cf + (size_t)(pot.s_f + pair_ij_index(s, o, pot.ntypes)) * FM_MAXB;
+        for (int q = 0; q < fp.NA; ++q) v += kbar[(size_t)s * fp.Dpad + (o * fp.NA + q) * fp.NN + a] * f[q];
       }
     }
-    // B-spline coefficient gradients -> (y, y'') table gradients of phi, rho, f, g
-    for (int s = 0; s < ns; ++s) {
-      if (s >= pot.s_U && s < pot.s_f) continue;  // U: table gradients already
-      const SplineGeom g = geom[s];
-      const int n = g.n;
-      const double H = g.step * g.step / 6.0, h2 = g.step * g.step;
-      const double *db = bgrad + (size_t)s * FM_MAXB;
-      double *y = tab + g.toff, *ypp = y + n;
-      // d_m+1 = y_m - H y''_m
-      for (int m = 0; m < n; ++m) {
-        y[m] += db[m + 1];
-        ypp[m] -= H * db[m + 1];
-      }
-      // d_0 = h2 y''_0 + 2 (y_0 - H y''_0) - (y_1 - H y''_1)
-      y[0] += 2.0 * db[0];
-      ypp[0] += (h2 - 2.0 * H) * db[0];
-      y[1] -= db[0];
-      ypp[1] += H * db[0];
-      // d_n+1 = h2 y''_n-1 + 2 (y_n-1 - H y''_n-1) - (y_n-2 - H y''_n-2)
-      y[n - 1] += 2.0 * db[n + 1];
-      ypp[n - 1] += (h2 - 2.0 * H) * db[n + 1];
-      y[n - 2] -= db[n + 1];
-      ypp[n - 2] += H * db[n + 1];
+    bgrad[i] = v;
+  }
+  __syncthreads();
+  // B-spline coefficient gradients -> (y, y'') table gradients of phi, rho, f, g
+  for (int s = threadIdx.x; s < ns; s += blockDim.x) {
+    if (s >= pot.s_U && s < pot.s_f) continue;  // U: table gradients already
+    const SplineGeom g = geom[s];
+    const int n = g.n;
+    const double H = g.step * g.step / 6.0, h2 = g.step * g.step;
+    const double *db = bgrad + (size_t)s * FM_MAXB;
+    double *y = tab + g.toff, *ypp = y + n;
+    // d_m+1 = y_m - H y''_m
+    for (int m = 0; m < n; ++m) {
+      y[m] += db[m + 1];
+      ypp[m] -= H * db[m + 1];
     }
+    // d_0 = h2 y''_0 + 2 (y_0 - H y''_0) - (y_1 - H y''_1)
+    y[0] += 2.0 * db[0];
+    ypp[0] += (h2 - 2.0 * H) * db[0];
+    y[1] -= db[0];
+    ypp[1] += H * db[0];
+    // d_n+1 = h2 y''_n-1 + 2 (y_n-1 - H y''_n-1) - (y_n-2 - H y''_n-2)
+    y[n - 1] += 2.0 * db[n + 1];
+    ypp[n - 1] += (h2 - 2.0 * H) * db[n + 1];
+    y[n - 2] -= db[n + 1];
+    ypp[n - 2] += H * db[n + 1];
   }
   __syncthreads();
   for (int e = threadIdx.x; e < stride; e += blockDim.x) out[(size_t)c * stride + e] = tab[e];

@@ -56,43 +56,42 @@ namespace mzb {
 
 // ---------------------------------------------------------- k_fm_kmat8
 
-// K8 and ke of one (type s, group gy): K_s[d][c] = c^{f(s,o)}_a w^{g(s)}_n in
-// FP64 (as k_fm_kmat), the column exponent over d, the digits.  Candidates
-// past ncand and features past D are zero.
-__global__ void __launch_bounds__(256) k_fm_kmat8(int ncand, DevPot pot, FmPlan fp,
-                                                  const double *__restrict__ coef64, signed char *__restrict__ K8,
-                                                  int *__restrict__ ke) {
-  __shared__ int se[FM8_NC];
-  const int s = blockIdx.x, gy = blockIdx.y;
-  const int nt = fp.nt;
-  auto kval = [&](int d, int cl) -> double {
-    const int c = gy * fp.CG + cl;
-    if (cl >= fp.CG || c >= ncand || d >= fp.D) return 0.0;
-    const int o = d / (fp.NA * fp.NN), a = (d / fp.NN) % fp.NA, nn = d % fp.NN;
-    const int fs = pot.s_f + pair_ij_index(s, o, pot.ntypes), gs = pot.s_g + s;
-    return coef64[((size_t)c * pot.nsplines + fs) * FM_MAXB + a] *
-           coef64[((size_t)c * pot.nsplines + gs) * FM_MAXB + nn];
-  };
-  // column maxima: one warp per candidate, lanes over the features
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int cl = warp; cl < FM8_NC; cl += blockDim.x >> 5) {
-    double m = 0.0;
-    for (int d = lane; d < FM8_D; d += 32) m = fmax(m, fabs(kval(d, cl)));
+// K8 and ke of one (type s, group gy, eight candidates): K_s[d][c] =
+// c^{f(s,o)}_a w^{g(s)}_n in FP64 (as k_fm_kmat), the column exponent over d,
+// the digits; a warp per candidate.  Candidates past ncand and features past D
+// are zero.  (A CTA for all 64 candidates of a type: 2 CTAs in all, 100 us.)
+constexpr int FM8_KC = 8;
+
+__global__ void __launch_bounds__(32 * FM8_KC) k_fm_kmat8(int ncand, DevPot pot, FmPlan fp,
+                                                          const double *__restrict__ coef64,
+                                                          signed char *__restrict__ K8, int *__restrict__ ke) {
+  const int s = blockIdx.x, gy = blockIdx.y, lane = threadIdx.x & 31, cl = blockIdx.z * FM8_KC + threadIdx.x / 32;
+  const int nt = fp.nt, c = gy * fp.CG + cl;
+  const bool live = cl < fp.CG && c < ncand;
+  double v[FM8_D / 32], m = 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) se[cl] = fm8_exponent(m);
+  for (int q = 0; q < FM8_D / 32; ++q) {
+    const int d = lane + 32 * q;
+    v[q] = 0.0;
+    if (live && d < fp.D) {
+      const int o = d / (fp.NA * fp.NN), a = (d / fp.NN) % fp.NA, nn = d % fp.NN;
+      const int fs = pot.s_f + pair_ij_index(s, o, pot.ntypes), gs = pot.s_g + s;
+      v[q] = coef64[((size_t)c * pot.nsplines + fs) * FM_MAXB + a] * coef64[((size_t)c * pot.nsplines + gs) * FM_MAXB + nn];
+    }
+    m = fmax(m, fabs(v[q]));
   }
-  __syncthreads();
-  if (threadIdx.x < FM8_NC) ke[((size_t)gy * nt + s) * FM8_NC + threadIdx.x] = se[threadIdx.x];
-  for (int idx = threadIdx.x; idx < FM8_NC * FM8_D; idx += blockDim.x) {
-    const int cl = idx % FM8_NC, d = idx / FM8_NC;
-    const long long v = llrint(ldexp(kval(d, cl), FM8_SHIFT - se[cl]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  const int e = fm8_exponent(m);
+  if (lane == 0) ke[((size_t)gy * nt + s) * FM8_NC + cl] = e;
+#pragma unroll
+  for (int q = 0; q < FM8_D / 32; ++q) {
+    const int d = lane + 32 * q;
     signed char dg[FM8_DIG];
-    digits256(v, dg);
-    const int kb = d >> 7;
+    digits256(llrint(ldexp(v[q], FM8_SHIFT - e)), dg);
     const uint32_t o = sw128_byte(cl, d & 127);
 #pragma unroll
-    for (int l = 0; l < FM8_DIG; ++l) K8[k8_block(gy, s, nt, kb, l) + o] = dg[l];
+    for (int l = 0; l < FM8_DIG; ++l) K8[k8_block(gy, s, nt, d >> 7, l) + o] = dg[l];
   }
 }
 
