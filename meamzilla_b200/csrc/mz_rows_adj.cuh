@@ -562,6 +562,7 @@ __global__ void __launch_bounds__(RADIAL_T)
       for (int it = it0[e / 4]; it < it0[e / 4 + 1]; ++it) acc[e] += isum[4 * it + (e & 3)];
     __syncthreads();
   }
+  __syncthreads();  // a CTA without a segment has only zeroed its sums
   double *out = part + ((size_t)cand * gridDim.x + blockIdx.x) * 4 * nb;
   for (int i = tid; i < 4 * nb; i += RADIAL_T) out[i] = acc[i];
 }

@@ -103,3 +103,24 @@ def test_candidates_of_a_batch_do_not_depend_on_it(style):
         b = one.objective(X[c:c + 1], MZ_FP64, errvec=True)
         assert a["obj"][c] == b["obj"][0]
         assert np.array_equal(a["errvec"][c], b["errvec"][0])
+
+
+def test_gradient_with_several_segments_per_cta():
+    """1.4 M slots: more segments of the radial sums than CTAs, so that some
+    CTAs take two and some none.  The gradient along five directions against
+    the tangent-linear oracle: rounding of sums over 4e4 atoms, 1e-11 of
+    |gradient| |direction|."""
+    from meamzilla_b200 import synth
+    from meamzilla_b200.potential import MZ_FP64, Evaluator
+    pot, db = _setup("eam/spline", 1, 5.5, seed=3, ncells=1200, rows=(40, 64))
+    assert db.stats()["npairs"] > 1.25e6
+    ev = Evaluator(db, pot, 1.0, 1.0, 0, max_candidates=1)
+    x = synth.perturbed(pot.coeffs(), 1, 0.01, seed=5)
+    orc = _oracle(ev)
+    g = [ev.objective_grad(x, MZ_FP64)[1][0] for _ in range(3)]
+    assert np.array_equal(g[0], g[1]) and np.array_equal(g[0], g[2])
+    rng = np.random.default_rng(2)
+    for _ in range(5):
+        d = rng.normal(size=x.size)
+        t = orc.tangent(x[0], d)[1]
+        assert abs(g[0] @ d - t) <= 1e-11 * np.linalg.norm(g[0]) * np.linalg.norm(d)
