@@ -623,10 +623,11 @@ bool fm_prepare(mz_ctx *ctx) {
   // second wave would run a fixed share of the blocks on a half-empty GPU);
   // launches of fewer candidates stage less and stay resident as well
   fm.smem_pre = fm_pre_smem(ctx->nsplines, 64, fp.nt, fp.NB, fp.ustride);
-  smem_attr(k_fm_adj_pre, fm.smem_pre);
+  smem_attr(k_fm_adj_pre<0>, fm.smem_pre);
+  smem_attr(k_fm_adj_pre<64>, fm.smem_pre);
   {
     int occ = 0;
-    ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fm_adj_pre, 256, fm.smem_pre), "occupancy");
+    ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fm_adj_pre<64>, 256, fm.smem_pre), "occupancy");
     fp.nctas_pre = std::max(1, std::min(fp.nblk, std::max(1, occ) * ctx->nsm));
   }
   fp.nctas_adj = std::max(1, std::min(fp.ntiles, ctx->nsm));
@@ -727,7 +728,8 @@ bool fm_prepare(mz_ctx *ctx) {
   smem_attr(k_fm_gemm_fwd<2>, fm_fwd_smem<2>(fp.Dpad));
   smem_attr(k_fm_gemm_fwd<4>, fm_fwd_smem<4>(fp.Dpad));
   smem_attr(k_fm_gemm_fwd<8>, fm_fwd_smem<8>(fp.Dpad));
-  smem_attr(k_fm_epi, fm_epi_smem(ctx->nsplines, fp.nt, fp.NB, 64));
+  smem_attr(k_fm_epi<0>, fm_epi_smem(ctx->nsplines, fp.nt, fp.NB, 64));
+  smem_attr(k_fm_epi<64>, fm_epi_smem(ctx->nsplines, fp.nt, fp.NB, 64));
   smem_attr(k_fm_gemm_adj<false>, fm_adj_smem(fp.Dpad, 64));
   if (fm.tc8) smem_attr(k_fm_gemm_adj<true>, fm_adj_smem(fp.Dpad, 64, true));
   fm.ready = true;
@@ -784,10 +786,10 @@ void enqueue_fm(mz_ctx *ctx, int n, double *d_obj, double *d_errvec, double *d_f
     // persistent CTAs, as many as are resident at once
     const size_t esm = fm_epi_smem(ns, fp.nt, fp.NB, CG);
     int occ = 0;
-    ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fm_epi, 256, esm), "occupancy");
+    auto epi = CG == 64 ? k_fm_epi<64> : k_fm_epi<0>;
+    ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, epi, 256, esm), "occupancy");
     const int eb = std::max(1, std::min(fp.nblk, std::max(1, occ) * ctx->nsm));
-    k_fm_epi<<<dim3(eb, G), 256, esm, st>>>(ctx->db, ctx->pot, ctx->d_geom,
-                                                                         ctx->d_tabs, fp, n);
+    epi<<<dim3(eb, G), 256, esm, st>>>(ctx->db, ctx->pot, ctx->d_geom, ctx->d_tabs, fp, n);
     ck(cudaGetLastError(), "k_fm_epi launch");
   }
   {
@@ -812,7 +814,8 @@ void enqueue_fm(mz_ctx *ctx, int n, double *d_obj, double *d_errvec, double *d_f
     ck(cudaMemsetAsync(fp.zmax, 0x80, sizeof(int) * (size_t)G * fm8_nspan(fp.Q) * FM8_NC, st), "memset");
   {
     Bracket b(ctx, MZ_K_FM_PRE);
-    k_fm_adj_pre<<<dim3(fp.nctas_pre, G), 256, fm_pre_smem(ns, CG, fp.nt, fp.NB, fp.ustride), st>>>(
+    auto pre = CG == 64 ? k_fm_adj_pre<64> : k_fm_adj_pre<0>;
+    pre<<<dim3(fp.nctas_pre, G), 256, fm_pre_smem(ns, CG, fp.nt, fp.NB, fp.ustride), st>>>(
         ctx->db, ctx->pot, ctx->d_geom, ctx->d_tabs, fp, n);
     ck(cudaGetLastError(), "k_fm_adj_pre launch");
   }
@@ -1200,7 +1203,24 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
         best.ctas = adj_ctas_for(ctx, 0, ctx->adj2_per_sm);
       }
       // the FP64 row kernels have no variants to time
-      const bool fixed = precision == MZ_FP64 && ctx->rows_ok && (!grad || ctx->radj.ready);
+      bool fixed = precision == MZ_FP64 && ctx->rows_ok && (!grad || ctx->radj.ready);
+      // Nor are the mixed row kernels' worth timing where the moment path beats
+      // their first variant by half: their best one is within 30 % of it, and
+      // the 18 trials of a large launch take seconds.
+      if (precision == MZ_MIXED && ctx->autotune == 1 && ctx->fm.eligible && ctx->fm_mode == 1 && fm_prepare(ctx)) {
+        const int64_t l0 = ctx->launches;
+        double t[2];
+        for (int fm = 0; fm < 2; ++fm) {
+          mz_ctx::Tune c = best;
+          c.fm = fm != 0;
+          apply_variant(ctx, c);
+          trial(ctx, n, d_params, precision, grad, -1);  // warm-up
+          t[fm] = trial(ctx, n, d_params, precision, grad, -1);
+        }
+        ctx->launches = l0;
+        best.fm = 1.5 * t[1] < t[0];
+        fixed = best.fm;
+      }
       if (ctx->autotune == 1 && !fixed) {
         const int64_t l0 = ctx->launches;
         apply_variant(ctx, best);
@@ -1248,7 +1268,7 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
       }
       // mixed meam/spline: the triplet-moment path, against the row kernels'
       // best (whole call), or always with MZ_FM=2
-      if (precision == MZ_MIXED && ctx->fm.eligible && ctx->fm_mode > 0 &&
+      if (!best.fm && precision == MZ_MIXED && ctx->fm.eligible && ctx->fm_mode > 0 &&
           (ctx->fm_mode == 2 || ctx->autotune == 1) && fm_prepare(ctx)) {
         if (ctx->fm_mode == 2) {
           best.fm = true;

@@ -482,12 +482,28 @@ __global__ void __launch_bounds__(NW * 32, 1) k_fm_gemm_fwd(FmPlan fp) {
 // frame (e1, e2), and the B-spline basis values (and d/dr) of phi, rho and f
 // at its shifts; and the pair splines' B-spline coefficients of the block's
 // atom type for the group's candidates.
+// A row's slots are staged sorted by (neighbour type, knot intervals): what a
+// slot needs of a candidate's coefficients depends on nothing else, so a walk
+// over the row keeps them in registers and reloads them at a change only (a
+// row of 41 slots has about 10).  Read slot by slot they made 99
+// shared-memory wavefronts per slot and warp of k_fm_epi, now 65.  With the
+// offsets of 64 candidates as immediates (CGT), 3.5 M slots x 64 candidates:
+// k_fm_epi 3996 -> 3020 us, k_fm_adj_pre 5980 -> 5190.  The pre pass's second
+// walk stays in listed order with one shared-memory addition per slot and
+// coefficient: adding a run's slots in registers first took it to 4020 us,
+// but moved the FP32 sums by 6.6e-9 of the gradient, three times what its
+// order of additions does by itself.  Prefetching the next block's rows of Y
+// into L2 changed nothing.
 constexpr int FM_ABLK = 4;   // atoms per block of the epilogues: 4 x 64 candidates fill 256 threads
 
 template <typename R>
 struct FmStage {
   int *satom, *arow;  // [FM_ABLK], [FM_ABLK + 1]
-  int *gs, *nbr, *tj, *kn;  // [BLOCK_SLOTS]
+  int *gs, *nbr, *pp;       // [BLOCK_SLOTS] global slot, neighbour, place in the row as listed
+  unsigned *key;            // [BLOCK_SLOTS] type << 24 | knots of f, rho, phi (each + 1)
+  unsigned *skey;           // [BLOCK_SLOTS] the keys as listed, before sorting
+  unsigned char *at;        // [BLOCK_SLOTS] the staged place (within the row) of the slot listed p-th
+  char4 *xe;                // [BLOCK_SLOTS] the slot's row exponents (FP32 stage of the integer contraction)
   int *ctype;         // type whose coefficients are staged (-1: none yet)
   float4 *uf;         // [BLOCK_SLOTS] (ux, uy, uz, 1/r)
   double *e;          // [BLOCK_SLOTS][6] e1 / r, e2 / r (FP32 stages keep e1, e2 as floats in the same space)
@@ -498,7 +514,7 @@ struct FmStage {
 
 template <typename R>
 __host__ __device__ inline size_t fm_stage_bytes(int nt, int NB, int CG) {
-  return sizeof(int) * (2 * FM_ABLK + 2 + 4 * BLOCK_SLOTS) + 16 + (sizeof(R) == 4 ? sizeof(float4) * BLOCK_SLOTS : 0) +
+  return sizeof(int) * (2 * FM_ABLK + 2 + (sizeof(R) == 4 ? 6 : 5) * BLOCK_SLOTS) + BLOCK_SLOTS + 16 + (sizeof(R) == 4 ? sizeof(float4) * BLOCK_SLOTS : 0) +
          sizeof(double4) * BLOCK_SLOTS + sizeof(double) * 6 * BLOCK_SLOTS + sizeof(R) * 24 * BLOCK_SLOTS +
          sizeof(R) * 3 * nt * NB * CG;
 }
@@ -523,9 +539,12 @@ __device__ __forceinline__ FmStage<R> fm_stage_carve(unsigned char *base, const 
   st.arow = ip + FM_ABLK;
   st.gs = st.arow + FM_ABLK + 1;
   st.nbr = st.gs + BLOCK_SLOTS;
-  st.tj = st.nbr + BLOCK_SLOTS;
-  st.kn = st.tj + BLOCK_SLOTS;
-  st.ctype = st.kn + BLOCK_SLOTS;
+  st.pp = st.nbr + BLOCK_SLOTS;
+  st.key = reinterpret_cast<unsigned *>(st.pp + BLOCK_SLOTS);
+  st.skey = st.key + BLOCK_SLOTS;
+  st.xe = reinterpret_cast<char4 *>(st.skey + BLOCK_SLOTS);
+  st.at = reinterpret_cast<unsigned char *>(st.skey + (sizeof(R) == 4 ? 2 : 1) * BLOCK_SLOTS);
+  st.ctype = reinterpret_cast<int *>(st.at + BLOCK_SLOTS);
   return st;
 }
 
@@ -558,17 +577,32 @@ __device__ int fm_stage_block(const DevDb &db, const DevPot &pot, const SplineGe
   const int nslot = st.arow[na];
   const int ti = db.atom_type[st.satom[0]];
   const int64_t Np = db.npairs;
-  for (int ql = tid; ql < nslot; ql += T) {
-    const int a = slot_owner(st.arow, na, ql);
-    const int i = st.satom[a], p = ql - st.arow[a];
+  for (int qi = tid; qi < nslot; qi += T) {
+    const int a = slot_owner(st.arow, na, qi);
+    const int64_t gs = db.pair_off[st.satom[a]] + (qi - st.arow[a]);
+    st.skey[qi] = (unsigned)db.atom_type[db.pair_nbr[gs]] << 24 | ((unsigned)db.pair_knot[gs] & 0xffffffu);
+  }
+  __syncthreads();
+  for (int qi = tid; qi < nslot; qi += T) {
+    const int a = slot_owner(st.arow, na, qi);
+    const int lo = st.arow[a], p = qi - lo, n = st.arow[a + 1] - lo;
+    const unsigned key = st.skey[qi];
+    int rank = 0;
+    for (int k = 0; k < n; ++k) {
+      const unsigned o = st.skey[lo + k];
+      rank += o < key || (o == key && k < p);
+    }
+    const int ql = lo + rank;
+    const int i = st.satom[a];
     const int64_t gs = db.pair_off[i] + p;
     const int j = db.pair_nbr[gs];
     st.gs[ql] = (int)gs;
     st.nbr[ql] = j;
-    const int tj = db.atom_type[j];
-    st.tj[ql] = tj;
-    const int kn = db.pair_knot[gs];
-    st.kn[ql] = kn;
+    st.pp[ql] = p;
+    st.key[ql] = key;
+    st.at[qi] = (unsigned char)rank;
+    if (sizeof(R) == 4 && fp.zmax) st.xe[ql] = *reinterpret_cast<const char4 *>(fp.xe + (fp.row0[i] + p) * 4);
+    const int tj = (int)(key >> 24), kn = (int)(key & 0xffffffu);
     if (sizeof(R) == 4) st.uf[ql] = make_float4(db.pair_uxf[gs], db.pair_uyf[gs], db.pair_uzf[gs], 1.f / db.pair_rf[gs]);
     st.ur[ql] = make_double4(db.pair_ux[gs], db.pair_uy[gs], db.pair_uz[gs], db.pair_r[gs]);
     const double *e = fp.E + (size_t)(fp.row0[i] + p) * 8;
@@ -617,11 +651,6 @@ __device__ int fm_stage_block(const DevDb &db, const DevPot &pot, const SplineGe
   return nslot;
 }
 
-// phi, rho, f (values and d/dr) of staged slot ql for candidate cl
-template <typename R>
-struct FmPairVals {
-  R phi, dphi, rho, drho, f, df;
-};
 // the staged basis of slot ql for pair function F: N0..N3, then their d/dr
 // (16-byte shared loads, the same address in every lane)
 __device__ __forceinline__ void fm_bas(const FmStage<float> &st, int ql, int F, float *b) {
@@ -630,56 +659,28 @@ __device__ __forceinline__ void fm_bas(const FmStage<float> &st, int ql, int F, 
   b[0] = x.x; b[1] = x.y; b[2] = x.z; b[3] = x.w;
   b[4] = y.x; b[5] = y.y; b[6] = y.z; b[7] = y.w;
 }
-__device__ __forceinline__ void fm_bas(const FmStage<double> &st, int ql, int F, double *b) {
-  const double2 *p = reinterpret_cast<const double2 *>(st.bas + (ql * 3 + F) * 8);
+// value (d = 0) or d/dr (d = 1) half of it
+__device__ __forceinline__ void fm_bas4(const FmStage<double> &st, int ql, int F, int d, double *b) {
+  const double2 *p = reinterpret_cast<const double2 *>(st.bas + (ql * 3 + F) * 8 + 4 * d);
+  const double2 x = p[0], y = p[1];
+  b[0] = x.x; b[1] = x.y; b[2] = y.x; b[3] = y.y;
+}
+
+// knot + 1 of pair function F in a slot's key (0: beyond its last knot)
+__device__ __forceinline__ int fm_key_knot(unsigned key, int F) { return (int)(key >> (8 * F)) & 0xff; }
+
+// the four coefficients that pair function F of a slot with this key uses
+template <typename R>
+__device__ __forceinline__ void fm_coef4(const FmStage<R> &st, const FmPlan &fp, int CG, unsigned key, int F, int cl,
+                                         R *c) {
+  const int k = max(fm_key_knot(key, F) - 1, 0);
+  const R *cf = st.coef + ((size_t)(F * fp.nt + (int)(key >> 24)) * fp.NB + k) * CG + cl;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const double2 x = p[i];
-    b[2 * i] = x.x;
-    b[2 * i + 1] = x.y;
-  }
+  for (int q = 0; q < 4; ++q) c[q] = cf[q * CG];
 }
-
-// value and d/dr of pair function F at staged slot ql for candidate cl
 template <typename R>
-__device__ __forceinline__ void fm_pair_val(const FmStage<R> &st, const FmPlan &fp, int ql, int cl, int F, int kn,
-                                            int tj, R &v, R &d) {
-  const int k = ((kn >> (8 * F)) & 0xff) - 1;
-  R bs[8];
-  fm_bas(st, ql, F, bs);
-  const int CG = fp.CG;
-  const R *cf = st.coef + ((size_t)(F * fp.nt + tj) * fp.NB + (k < 0 ? 0 : k)) * CG + cl;
-  const R c0 = cf[0], c1 = cf[CG], c2 = cf[2 * CG], c3 = cf[3 * CG];
-  v = bs[0] * c0 + bs[1] * c1 + bs[2] * c2 + bs[3] * c3;  // zero basis where k < 0
-  d = bs[4] * c0 + bs[5] * c1 + bs[6] * c2 + bs[7] * c3;
-}
-
-// only the value (d = 0) or only d/dr (d = 1) of pair function F
-template <typename R>
-__device__ __forceinline__ R fm_pair_one(const FmStage<R> &st, const FmPlan &fp, int ql, int cl, int F, int kn, int tj,
-                                         int d) {
-  const int k = ((kn >> (8 * F)) & 0xff) - 1;
-  const R *bs = st.bas + (ql * 3 + F) * 8 + 4 * d;
-  R b[4];
-  if (sizeof(R) == 4) {
-    const float4 x = *reinterpret_cast<const float4 *>(bs);
-    b[0] = x.x; b[1] = x.y; b[2] = x.z; b[3] = x.w;
-  } else {
-    const double2 x = reinterpret_cast<const double2 *>(bs)[0], y = reinterpret_cast<const double2 *>(bs)[1];
-    b[0] = x.x; b[1] = x.y; b[2] = y.x; b[3] = y.y;
-  }
-  const int CG = fp.CG;
-  const R *cf = st.coef + ((size_t)(F * fp.nt + tj) * fp.NB + (k < 0 ? 0 : k)) * CG + cl;
-  return b[0] * cf[0] + b[1] * cf[CG] + b[2] * cf[2 * CG] + b[3] * cf[3 * CG];  // zero basis where k < 0
-}
-
-template <typename R>
-__device__ __forceinline__ FmPairVals<R> fm_pair_vals(const FmStage<R> &st, const FmPlan &fp, int ql, int cl) {
-  R v[3], d[3];
-  const int kn = st.kn[ql], tj = st.tj[ql];
-#pragma unroll
-  for (int F = 0; F < 3; ++F) fm_pair_val(st, fp, ql, cl, F, kn, tj, v[F], d[F]);
-  return FmPairVals<R>{v[0], d[0], v[1], d[1], v[2], d[2]};
+__device__ __forceinline__ R fm_dot4(const R *b, const R *c) {  // zero basis beyond the last knot
+  return b[0] * c[0] + b[1] * c[1] + b[2] * c[2] + b[3] * c[3];
 }
 
 // ---------------------------------------------------------------- k_fm_epi
@@ -698,13 +699,15 @@ __host__ __device__ inline size_t fm_epi_smem(int nsplines, int nt, int NB, int 
   return ((fm_stage_bytes<double>(nt, NB, CG) + 15) & ~size_t(15)) + sizeof(SplineGeom) * (size_t)nsplines;
 }
 
+// CGT: the candidates per group where they are 64 (offsets become immediates), else 0.
+template <int CGT>
 __global__ void __launch_bounds__(256) k_fm_epi(DevDb db, DevPot pot, const SplineGeom *__restrict__ geom,
                                                const double *__restrict__ tabs, FmPlan fp, int ncand) {
   extern __shared__ __align__(16) unsigned char fm_raw[];
   const FmStage<double> st = fm_stage_carve<double>(fm_raw, fp);
   SplineGeom *sg = reinterpret_cast<SplineGeom *>(
       fm_raw + ((fm_stage_bytes<double>(fp.nt, fp.NB, fp.CG) + 15) & ~size_t(15)));
-  const int gy = blockIdx.y, CG = fp.CG, N = db.natoms;
+  const int gy = blockIdx.y, CG = CGT ? CGT : fp.CG, N = db.natoms;
   const int tid = threadIdx.x, T = blockDim.x;
   for (int s = tid; s < pot.nsplines; s += T) sg[s] = geom[s];
   if (tid == 0) *st.ctype = -1;
@@ -724,14 +727,29 @@ __global__ void __launch_bounds__(256) k_fm_epi(DevDb db, DevPot pot, const Spli
       const int i = st.satom[a], lo = st.arow[a], n = st.arow[a + 1] - lo;
       const float *Yq = fp.Y + ((size_t)gy * fp.Q + fp.row0[i]) * 3 * CG + cl;
       double rho = 0.0, epair = 0.0;
-#pragma unroll 4
-      for (int p = 0; p < n; ++p) {
-        const int ql = lo + p, kn = st.kn[ql], tj = st.tj[ql];
-        const double phi = fm_pair_one<double>(st, fp, ql, cl, 0, kn, tj, 0);
-        const double rv = fm_pair_one<double>(st, fp, ql, cl, 1, kn, tj, 0);
-        const double fv = fm_pair_one<double>(st, fp, ql, cl, 2, kn, tj, 0);
-        rho += rv + 0.5 * fv * (double)Yq[(size_t)p * 3 * CG];
-        epair += 0.5 * phi;
+      unsigned prev = ~0u;
+      double cv[3][4];
+      // slots in batches of FM_PBW, every load of a batch first
+      for (int p0 = 0; p0 < n; p0 += FM_PBW) {
+        float gv[FM_PBW];
+#pragma unroll
+        for (int j = 0; j < FM_PBW; ++j) gv[j] = Yq[(size_t)st.pp[lo + min(p0 + j, n - 1)] * 3 * CG];
+#pragma unroll
+        for (int j = 0; j < FM_PBW; ++j) {
+          if (p0 + j >= n) break;
+          const int ql = lo + p0 + j;
+          const unsigned key = st.key[ql];
+          if (key != prev) {
+            prev = key;
+#pragma unroll
+            for (int F = 0; F < 3; ++F) fm_coef4<double>(st, fp, CG, key, F, cl, cv[F]);
+          }
+          double b[3][4];
+#pragma unroll
+          for (int F = 0; F < 3; ++F) fm_bas4(st, ql, F, 0, b[F]);
+          rho += fm_dot4(b[1], cv[1]) + 0.5 * fm_dot4(b[2], cv[2]) * (double)gv[j];
+          epair += 0.5 * fm_dot4(b[0], cv[0]);
+        }
       }
       const double w = db.cell_w[db.atom_cell[i]];
       double pen = 0.0, rt = rho;
@@ -745,12 +763,13 @@ __global__ void __launch_bounds__(256) k_fm_epi(DevDb db, DevPot pot, const Spli
       const PointEval U = spl_point(tc, gU, rt);
       const double dF = U.grad;
       double F[3] = {0, 0, 0}, S[6] = {0, 0, 0, 0, 0, 0};
+      prev = ~0u;
       // slots in batches of FM_PB, every load of a batch before its stores
       for (int p0 = 0; p0 < n; p0 += FM_PB) {
         float yv[FM_PB][3];
 #pragma unroll
         for (int j = 0; j < FM_PB; ++j) {
-          const float *yp = Yq + (size_t)min(p0 + j, n - 1) * 3 * CG;
+          const float *yp = Yq + (size_t)st.pp[lo + min(p0 + j, n - 1)] * 3 * CG;
           yv[j][0] = yp[0];
           yv[j][1] = yp[CG];
           yv[j][2] = yp[2 * CG];
@@ -760,20 +779,28 @@ __global__ void __launch_bounds__(256) k_fm_epi(DevDb db, DevPot pot, const Spli
         const int p = p0 + j;
         if (p >= n) break;
         const int ql = lo + p;
-        FmPairVals<double> v;
-        {
-          const int kn = st.kn[ql], tj = st.tj[ql];
-          v.dphi = fm_pair_one<double>(st, fp, ql, cl, 0, kn, tj, 1);
-          v.drho = fm_pair_one<double>(st, fp, ql, cl, 1, kn, tj, 1);
-          fm_pair_val<double>(st, fp, ql, cl, 2, kn, tj, v.f, v.df);
+        const unsigned key = st.key[ql];
+        if (key != prev) {
+          prev = key;
+#pragma unroll
+          for (int F = 0; F < 3; ++F) fm_coef4<double>(st, fp, CG, key, F, cl, cv[F]);
         }
+        double b[4];
+        fm_bas4(st, ql, 0, 1, b);
+        const double dphi = fm_dot4(b, cv[0]);
+        fm_bas4(st, ql, 1, 1, b);
+        const double drho = fm_dot4(b, cv[1]);
+        fm_bas4(st, ql, 2, 0, b);
+        const double f = fm_dot4(b, cv[2]);
+        fm_bas4(st, ql, 2, 1, b);
+        const double df = fm_dot4(b, cv[2]);
         const double G = yv[j][0], Y1 = yv[j][1], Y2 = yv[j][2];  // FP32 sums, FP64 arithmetic
         const double *e = st.e + ql * 6;
         const int64_t gs = st.gs[ql];
         const double4 ur = st.ur[ql];
         const double rr = ur.w, dx = ur.x, dy = ur.y, dz = ur.z;
-        const double A = 0.5 * v.dphi + dF * (v.drho + v.df * G);
-        const double B = dF * v.f;  // the staged frames carry the 1 / r
+        const double A = 0.5 * dphi + dF * (drho + df * G);
+        const double B = dF * f;  // the staged frames carry the 1 / r
         const double Vx = dx * A + B * (e[0] * Y1 + e[3] * Y2);
         const double Vy = dy * A + B * (e[1] * Y1 + e[4] * Y2);
         const double Vz = dz * A + B * (e[2] * Y1 + e[5] * Y2);
@@ -968,10 +995,11 @@ __host__ __device__ inline size_t fm_pre_smem(int nsplines, int CG, int nt, int 
   return b;
 }
 
+template <int CGT>
 __global__ void __launch_bounds__(256, 2) k_fm_adj_pre(DevDb db, DevPot pot, const SplineGeom *__restrict__ geom,
                                                       const double *__restrict__ tabs, FmPlan fp, int ncand) {
   extern __shared__ __align__(16) unsigned char fm_raw[];
-  const int gy = blockIdx.y, CG = fp.CG, N = db.natoms, NC = db.ncells;
+  const int gy = blockIdx.y, CG = CGT ? CGT : fp.CG, N = db.natoms, NC = db.ncells;
   const int tid = threadIdx.x, T = blockDim.x;
   const FmStage<float> st = fm_stage_carve<float>(fm_raw, fp);
   size_t off = (fm_stage_bytes<float>(fp.nt, fp.NB, CG) + 15) & ~size_t(15);
@@ -1055,30 +1083,29 @@ __global__ void __launch_bounds__(256, 2) k_fm_adj_pre(DevDb db, DevPot pot, con
       // the integer adjoint's operand Z = 2^(e_q - 30) dL/dY: its exponent
       // bound per (span of FM8_SPAN 128-slot tiles, candidate),
       // |v| < 2^(field - 126), kept as the running maximum of the span
-      int64_t zspan = -1;
-      int zexp = -1000;
+      // (a row meets one boundary of spans at most: listed slots before pz and from it on)
+      const int64_t zs = q0 >> (7 + FM8_SPAN_LOG);
+      const int pz = (int)min((int64_t)n, ((zs + 1) << (7 + FM8_SPAN_LOG)) - q0);
+      int z0 = -100000, z1 = -100000;
       // FP32 exponent field of v plus e_q (a value's bound before the
       // constant -126 - 30), far below every bound for v = 0
       auto zfield = [](float v, int eq) { return v != 0.f ? (int)((__float_as_uint(v) >> 23) & 255) + eq : -100000; };
-      auto zbound = [&](int64_t q, int fe) {
-        const int64_t sp = q >> (7 + FM8_SPAN_LOG);
-        if (sp != zspan) {
-          if (zspan >= 0 && zexp > -1000) atomicMax(fp.zmax + ((size_t)gy * nspan8 + zspan) * 64 + cl, zexp);
-          zspan = sp;
-          zexp = -1000;
-        }
-        zexp = max(zexp, fe - 126 - FM8_SHIFT);
+      auto zbound = [&](int p, int fe) {
+        if (p < pz) z0 = max(z0, fe);
+        else z1 = max(z1, fe);
       };
       auto zflush = [&]() {
-        if (zspan >= 0 && zexp > -1000) atomicMax(fp.zmax + ((size_t)gy * nspan8 + zspan) * 64 + cl, zexp);
-        zspan = -1;
-        zexp = -1000;
+        int *zm = fp.zmax + ((size_t)gy * nspan8 + zs) * 64 + cl;
+        if (z0 - 126 - FM8_SHIFT > -1000) atomicMax(zm, z0 - 126 - FM8_SHIFT);
+        if (z1 - 126 - FM8_SHIFT > -1000) atomicMax(zm + 64, z1 - 126 - FM8_SHIFT);
       };
       const float dF = (float)U.grad;
       // ---- pass 1: K_i, dL/dY1 and dL/dY2 (they do not depend on chi_i), and
       // per slot (a_p, G_p, U' (Lambda.e1 Y1 + Lambda.e2 Y2) / r_p) for pass 2,
       // kept as FP32 in the slot's own Y words (Y is not read again)
       double K = 0.0;
+      unsigned prev = ~0u;
+      float cv[3][4];
       // slots in batches of FM_PB: every load of a batch is issued before its
       // stores (the stores go to the same arrays, so the compiler would
       // otherwise keep each slot's loads behind the previous slot's stores)
@@ -1087,22 +1114,30 @@ __global__ void __launch_bounds__(256, 2) k_fm_adj_pre(DevDb db, DevPot pot, con
         float lj[FM_PB][3];
 #pragma unroll
         for (int j = 0; j < FM_PB; ++j) {
-          const int p = min(p0 + j, n - 1);  // past the row: the last slot again, not used
-          const float *yp = Yq + (size_t)p * 3 * CG;
+          const int ql = lo + min(p0 + j, n - 1);  // past the row: the last slot again, not used
+          const float *yp = Yq + (size_t)st.pp[ql] * 3 * CG;
           yv[j][0] = yp[0];
           yv[j][1] = yp[CG];
           yv[j][2] = yp[2 * CG];
-          const float *Lj = fp.lamf + ((size_t)gy * N + st.nbr[lo + p]) * 3 * CG + cl;
+          const float *Lj = fp.lamf + ((size_t)gy * N + st.nbr[ql]) * 3 * CG + cl;
           lj[j][0] = __ldg(Lj);
           lj[j][1] = __ldg(Lj + CG);
           lj[j][2] = __ldg(Lj + 2 * CG);
         }
 #pragma unroll
         for (int j = 0; j < FM_PB; ++j) {
-          const int p = p0 + j;
-          if (p >= n) break;
-          const int ql = lo + p;
-          const FmPairVals<float> v = fm_pair_vals<float>(st, fp, ql, cl);
+          if (p0 + j >= n) break;
+          const int ql = lo + p0 + j, p = st.pp[ql];
+          const unsigned key = st.key[ql];
+          if (key != prev) {
+            prev = key;
+            fm_coef4<float>(st, fp, CG, key, 1, cl, cv[1]);
+            fm_coef4<float>(st, fp, CG, key, 2, cl, cv[2]);
+          }
+          float b1[8], b2[8];
+          fm_bas(st, ql, 1, b1);
+          fm_bas(st, ql, 2, b2);
+          const float drho = fm_dot4(b1 + 4, cv[1]), f = fm_dot4(b2, cv[2]), df = fm_dot4(b2 + 4, cv[2]);
           float *yp = Yq + (size_t)p * 3 * CG;
           const float G = yv[j][0], Y1 = yv[j][1], Y2 = yv[j][2];
           const float4 u = st.uf[ql];
@@ -1113,8 +1148,8 @@ __global__ void __launch_bounds__(256, 2) k_fm_adj_pre(DevDb db, DevPot pot, con
           const float l1 = lx * e[0] + ly * e[1] + lz * e[2], l2 = lx * e[3] + ly * e[4] + lz * e[5];
           const float t12 = (l1 * Y1 + l2 * Y2) * u.w;
           // the slot's term in FP32, the atom's sum in FP64
-          K += (double)(ap * (v.drho + v.df * G) + v.f * t12);
-          const float B = dF * v.f * u.w, y1 = B * l1, y2 = B * l2;
+          K += (double)(ap * (drho + df * G) + f * t12);
+          const float B = dF * f * u.w, y1 = B * l1, y2 = B * l2;
           float *yb = Ybq + (size_t)p * 3 * CG;
           yb[CG] = y1;
           yb[2 * CG] = y2;
@@ -1122,8 +1157,8 @@ __global__ void __launch_bounds__(256, 2) k_fm_adj_pre(DevDb db, DevPot pot, con
           yp[CG] = G;
           yp[2 * CG] = dF * t12;
           if (fp.zmax) {
-            const char4 eq = *reinterpret_cast<const char4 *>(fp.xe + (q0 + p) * 4);
-            zbound(q0 + p, max(zfield(y1, eq.y), zfield(y2, eq.z)));
+            const char4 eq = st.xe[ql];
+            zbound(p, max(zfield(y1, eq.y), zfield(y2, eq.z)));
           }
         }
       }
@@ -1142,39 +1177,31 @@ __global__ void __launch_bounds__(256, 2) k_fm_adj_pre(DevDb db, DevPot pot, con
           svv[j] = yp[2 * CG];
         }
 #pragma unroll
-      for (int j = 0; j < FM_PBW; ++j) {
-        const int p = p0 + j;
-        if (p >= n) break;
-        const int ql = lo + p;
-        const float ap = aGv[j].x, G = aGv[j].y, sv = svv[j];
-        const int kn = st.kn[ql], tj = st.tj[ql];
-        float bs[3][8];
+        for (int j = 0; j < FM_PBW; ++j) {
+          const int p = p0 + j;
+          if (p >= n) break;
+          const int ql = lo + st.at[lo + p];
+          const float ap = aGv[j].x, G = aGv[j].y, sv = svv[j];
+          const unsigned key = st.key[ql];
+          fm_coef4<float>(st, fp, CG, key, 2, cl, cv[2]);
+          float bs[3][8];
 #pragma unroll
-        for (int F = 0; F < 3; ++F) fm_bas(st, ql, F, bs[F]);
-        float f, df;
-        {
-          const int k = ((kn >> 16) & 0xff) - 1;
-          const float *cf = st.coef + ((size_t)(2 * fp.nt + tj) * fp.NB + (k < 0 ? 0 : k)) * CG + cl;
-          const float c0 = cf[0], c1 = cf[CG], c2 = cf[2 * CG], c3 = cf[3 * CG];
-          f = bs[2][0] * c0 + bs[2][1] * c1 + bs[2][2] * c2 + bs[2][3] * c3;  // zero basis where k < 0
-          df = bs[2][4] * c0 + bs[2][5] * c1 + bs[2][6] * c2 + bs[2][7] * c3;
-        }
-        const float y0 = 0.5f * f * ch + ap * dF * df;
-        Ybq[(size_t)p * 3 * CG] = y0;
-        if (fp.zmax) zbound(q0 + p, zfield(y0, (int)fp.xe[(q0 + p) * 4]));
-        const float wv[3] = {0.5f * epsf, ch, 0.5f * ch * G + sv};
-        const float wd[3] = {0.5f * ap, dF * ap, dF * ap * G};
+          for (int F = 0; F < 3; ++F) fm_bas(st, ql, F, bs[F]);
+          const float f = fm_dot4(bs[2], cv[2]), df = fm_dot4(bs[2] + 4, cv[2]);
+          const float y0 = 0.5f * f * ch + ap * dF * df;
+          Ybq[(size_t)p * 3 * CG] = y0;
+          if (fp.zmax) zbound(p, zfield(y0, (int)st.xe[ql].x));
+          const float wv[3] = {0.5f * epsf, ch, 0.5f * ch * G + sv};
+          const float wd[3] = {0.5f * ap, dF * ap, dF * ap * G};
 #pragma unroll
-        for (int F = 0; F < 3; ++F) {
-          const int k = ((kn >> (8 * F)) & 0xff) - 1;
-          if (k < 0) continue;
-          float *pe = pacc + ((size_t)(F * fp.nt + tj) * fp.NB + k) * CG + cl;
-          atomicAdd(pe, wv[F] * bs[F][0] + wd[F] * bs[F][4]);
-          atomicAdd(pe + CG, wv[F] * bs[F][1] + wd[F] * bs[F][5]);
-          atomicAdd(pe + 2 * CG, wv[F] * bs[F][2] + wd[F] * bs[F][6]);
-          atomicAdd(pe + 3 * CG, wv[F] * bs[F][3] + wd[F] * bs[F][7]);
+          for (int F = 0; F < 3; ++F) {
+            const int k = fm_key_knot(key, F) - 1;
+            if (k < 0) continue;
+            float *pe = pacc + ((size_t)(F * fp.nt + (int)(key >> 24)) * fp.NB + k) * CG + cl;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) atomicAdd(pe + q * CG, wv[F] * bs[F][q] + wd[F] * bs[F][4 + q]);
+          }
         }
-      }
       }
       if (fp.zmax) zflush();
     }
