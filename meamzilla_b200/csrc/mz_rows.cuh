@@ -368,6 +368,7 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
         }
         __syncwarp();
         auto pass = [&](const RowSpl *a, auto weight) {
+          if (nw == 0) return;  // no row is staged: the shared rows hold anything
           // as many slots a lane as the warp's longest row needs
           auto go = [&](auto cl) {
             constexpr bool CL = decltype(cl)::value;

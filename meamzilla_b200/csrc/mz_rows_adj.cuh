@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(32 * RADJ_MAXW, 1)
         ruzw[l + s * LPA].y += 0.5 * chi * f[s];
       }
       __syncwarp();
-      double dk[SPL];
+      double dk[SPL] = {};
       const RowSpl *a = spl + pot.s_g + ti * L.ntab;
       auto go = [&](auto cl) {
         constexpr bool CL = decltype(cl)::value;
@@ -385,8 +385,12 @@ __global__ void __launch_bounds__(32 * RADJ_MAXW, 1)
         else if (nw > LPA) radj_pass<CL, 2, LPA, GM>(row, nw, l, u, f, alo, ahi, a, pot, tj, tab, L.np, dk);
         else radj_pass<CL, 1, LPA, GM>(row, nw, l, u, f, alo, ahi, a, pot, tj, tab, L.np, dk);
       };
-      if (pot.ang_cover) go(std::integral_constant<bool, false>{});
-      else go(std::integral_constant<bool, true>{});
+      if (nw == 0) {  // no row is staged: the shared rows hold anything
+      } else if (pot.ang_cover) {
+        go(std::integral_constant<bool, false>{});
+      } else {
+        go(std::integral_constant<bool, true>{});
+      }
 #pragma unroll
       for (int s = 0; s < SPL; ++s) {
         const int p = l + s * LPA;

@@ -13,7 +13,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def _setup(style, ntypes, rcut, seed, ncells=3, gspan=(-1.0, 1.0), rows=None):
+def _setup(style, ntypes, rcut, seed, ncells=3, gspan=(-1.0, 1.0), rows=None, isolated=1):
     """Database whose longest row is in (rows[0], rows[1]]: cells of one shape
     at a density that grows until it is."""
     from meamzilla_b200 import synth
@@ -37,9 +37,10 @@ def _setup(style, ntypes, rcut, seed, ncells=3, gspan=(-1.0, 1.0), rows=None):
             pos = frac[:n] @ L + rng.uniform(-0.05, 0.05, (n, 3))
             cells.append(synth.Cell(lattice=L, types=rng.integers(0, ntypes, n), pos=pos,
                                     force0=rng.normal(0, 0.3, (n, 3)), energy0=-1.0, stress0=rng.normal(0, 1e-3, 6)))
-        # an isolated atom: an empty row
-        cells.append(synth.Cell(lattice=np.eye(3) * 30.0, types=np.zeros(1, dtype=int), pos=np.zeros((1, 3)),
-                                force0=np.zeros((1, 3))))
+        # isolated atoms: empty rows
+        for k in range(isolated):
+            cells.insert(len(cells) - 2 * k, synth.Cell(
+                lattice=np.eye(3) * 30.0, types=np.zeros(1, dtype=int), pos=np.zeros((1, 3)), force0=np.zeros((1, 3))))
         db = Database.from_cells(cells, pot)
         if rows is None or db.stats()["max_row"] > rows[0]:
             break
@@ -121,6 +122,28 @@ def test_gradient_with_several_segments_per_cta():
     assert np.array_equal(g[0], g[1]) and np.array_equal(g[0], g[2])
     rng = np.random.default_rng(2)
     for _ in range(5):
+        d = rng.normal(size=x.size)
+        t = orc.tangent(x[0], d)[1]
+        assert abs(g[0] @ d - t) <= 1e-11 * np.linalg.norm(g[0]) * np.linalg.norm(d)
+
+
+@pytest.mark.parametrize("style,rcut,rows", [("meam/spline", 7.0, (64, 128)), ("meam/spline", 4.0, (8, 32)),
+                                             ("gmeam/spline", 7.0, (64, 128))])
+def test_empty_rows_between_others(style, rcut, rows):
+    """Empty rows that a warp takes after others, whose staged slots they must
+    not read: 90 cells of 30 to 32 atoms and 40 isolated atoms.  The gradient
+    along three directions against the tangent-linear oracle: rounding of sums
+    over 3e3 atoms, 1e-11 of |gradient| |direction|."""
+    from meamzilla_b200 import synth
+    from meamzilla_b200.potential import MZ_FP64, Evaluator
+    pot, db = _setup(style, 1, rcut, seed=3, ncells=90, rows=rows, isolated=40)
+    ev = Evaluator(db, pot, 1.0, 1.0, 0, max_candidates=1)
+    x = synth.perturbed(pot.coeffs(), 1, 0.01, seed=5)
+    orc = _oracle(ev)
+    obj, g = ev.objective_grad(x, MZ_FP64)
+    assert np.array_equal(obj, ev.objective(x, MZ_FP64))
+    rng = np.random.default_rng(2)
+    for _ in range(3):
         d = rng.normal(size=x.size)
         t = orc.tangent(x[0], d)[1]
         assert abs(g[0] @ d - t) <= 1e-11 * np.linalg.norm(g[0]) * np.linalg.norm(d)
