@@ -638,7 +638,7 @@ bool fm_prepare(mz_ctx *ctx) {
   };
   Need need[] = {
       {ctx->d_aux, sizeof(double) * C * aux_rows * Np, 2 * sizeof(float) * G * Q * 3 * CG},  // Y, Yb
-      {ctx->d_V, sizeof(double) * C * 3 * Np, sizeof(double) * Cp * Np * 3},                   // V
+      {ctx->d_V, sizeof(double) * C * 4 * Np, sizeof(double) * Cp * Np * 3},                   // V
       {ctx->d_aout, sizeof(double) * C * AO_COUNT * N, sizeof(double) * Cp * AO_COUNT * N},    // aoutF
       {ctx->d_lam, sizeof(double) * C * 3 * N, sizeof(float) * Cp * 3 * N},                    // lamf
       {ctx->d_seeds, sizeof(double) * C * CS_COUNT * NC, sizeof(double) * Cp * CS_COUNT * NC}, // seedF
@@ -893,7 +893,7 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
   if (!d_obj) return;
   {
     Bracket b(ctx, MZ_K_GATHER);
-    k_force<<<dim3((unsigned)(((int64_t)ctx->natoms * FORCE_LANES + 255) / 256), n), 256, 0, st>>>(
+    k_force<4><<<dim3((unsigned)(((int64_t)ctx->natoms * FORCE_LANES + 255) / 256), n), 256, 0, st>>>(
         ctx->db, ctx->d_V, ctx->d_aout, d_forces, d_errvec, ctx->esize, grad ? ctx->d_lam : nullptr);
     ck(cudaGetLastError(), "k_force launch");
   }
@@ -1544,6 +1544,7 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     d.ncells = db.ncells;
     d.natoms = N;
     d.npairs = Np;
+    d.vs = 4;
     d.cell_atom0 = dupload(ctx, db.cell_atom0.data(), db.cell_atom0.size());
     d.cell_vol = dupload(ctx, db.cell_vol.data(), db.cell_vol.size());
     d.cell_w = dupload(ctx, db.cell_weight.data(), db.cell_weight.size());
@@ -1889,7 +1890,7 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     size_t freeb = 0, totalb = 0;
     ck(cudaMemGetInfo(&freeb, &totalb), "cudaMemGetInfo");
     const size_t per_cand =
-        sizeof(double) * ((size_t)(3 + (meam ? dp.aux_rows : 0)) * Np + (size_t)(AO_COUNT + 3 + 3) * N +
+        sizeof(double) * ((size_t)(4 + (meam ? dp.aux_rows : 0)) * Np + (size_t)(AO_COUNT + 3 + 3) * N +
                           (size_t)ctx->esize + (size_t)(8 + 1 + CS_COUNT) * db.ncells + 2 * (size_t)stride + ctx->pstride +
                           (size_t)ctx->adj_ctas_max * stride * (1 + ADJ_WARPS) + (size_t)2049 * stride +
                           2 * (size_t)ctx->P + 1) +
@@ -1901,7 +1902,7 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     ctx->d_params = dalloc<double>(ctx, C * ctx->P);
     ctx->d_tabs = dalloc<double>(ctx, C * stride);
     ctx->d_ptabs = dalloc<double>(ctx, C * ctx->pstride);
-    ctx->d_V = dalloc<double>(ctx, C * 3 * Np);
+    ctx->d_V = dalloc<double>(ctx, C * 4 * Np);
     ctx->d_aout = dalloc<double>(ctx, C * AO_COUNT * N);
     ctx->d_forces = dalloc<double>(ctx, C * 3 * N);
     ctx->d_cellobj = dalloc<double>(ctx, C * db.ncells);
@@ -2372,6 +2373,7 @@ extern "C" mz_status mz_objective_noalloc(const mz_db *dbh, const mz_pot *poth, 
     d.ncells = NC;
     d.natoms = N;
     d.npairs = Np;
+    d.vs = 3;
     d.nblocks = nblocks;
     d.cell_atom0 = (const int *)D(o_atom0);
     d.cell_vol = (const double *)D(o_vol);
@@ -2408,7 +2410,7 @@ extern "C" mz_status mz_objective_noalloc(const mz_db *dbh, const mz_pot *poth, 
     else
       k_atoms<false, double, false><<<ga, BLOCK_SLOTS, sa>>>(d, dp, dgeom, tabs, ptabs, V, aout, nullptr);
     ck(cudaGetLastError(), "k_atoms launch");
-    k_force<<<dim3((unsigned)(((int64_t)N * FORCE_LANES + 255) / 256), 1), 256>>>(d, V, aout, dforces, nullptr, 0,
+    k_force<3><<<dim3((unsigned)(((int64_t)N * FORCE_LANES + 255) / 256), 1), 256>>>(d, V, aout, dforces, nullptr, 0,
                                                                                   nullptr);
     ck(cudaGetLastError(), "k_force launch");
     // k_cells' counter: the atoms' own-force sums are read by now

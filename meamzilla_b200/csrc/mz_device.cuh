@@ -6,6 +6,15 @@
 
 namespace mzb {
 
+// 32-byte records (x, y, z, -), aligned: one load and one store each
+__device__ __forceinline__ void load_vec4(const double *p, double &x, double &y, double &z) {
+  [[maybe_unused]] double w;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x), "=d"(y), "=d"(z), "=d"(w) : "l"(p));
+}
+__device__ __forceinline__ void store_vec4(double *p, double x, double y, double z) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" : : "l"(p), "d"(x), "d"(y), "d"(z), "d"(0.0) : "memory");
+}
+
 constexpr int MAX_SPLINES = 64;     // splines in one potential (8 types MEAM: 36+8+8+36+8)
 constexpr int BLOCK_SLOTS = 256;    // pair slots (threads) of one atom block
 constexpr int BLOCK_ATOMS = 64;     // atoms of one atom block
@@ -46,6 +55,7 @@ struct DevDb {
   const double *force0;           // [3N]
   const int *pair_off;            // [N+1]
   const int *in_off, *in_slot;    // incoming lists
+  int vs;                         // doubles per slot of the pair forces V: 4 (32-byte records), or 3 packed
   // pairs
   const int *pair_nbr;
   const double *pair_r, *pair_ux, *pair_uy, *pair_uz;

@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(BLOCK_SLOTS, JM ? 2 : sizeof(R) == 4 ? 4 : 3)
     Vx += ux * cu;
     Vy += uy * cu;
     Vz += uz * cu;
-    double *Vc = Vout + (size_t)cand * 3 * Np + 3 * gs;  // (x, y, z) per slot
+    double *Vc = Vout + ((size_t)cand * Np + gs) * db.vs;  // (x, y, z) per slot
     Vc[0] = Vx;
     Vc[1] = Vy;
     Vc[2] = Vz;
@@ -640,24 +640,40 @@ __global__ void __launch_bounds__(BLOCK_SLOTS, JM ? 2 : sizeof(R) == 4 ? 4 : 3)
 // and, for the adjoint, lambda_i = dF/dF_i = 2 w e_i.  Eight lanes per atom:
 // a lane per atom walked its 16 to 60 incoming slots one dependent read after
 // another (16 us for 21 k atoms of 16 slots, one candidate; this takes 6).
+// The reads are scattered, and three 8-byte loads a slot kept the L1 busy 97 %
+// of the time: V is stored as records of 32 bytes that one load fetches (18 k
+// atoms of 42 slots, 128 candidates: 592 -> 558 us, 5.2 TB/s; k_rows, which
+// writes them without staging, 1408 -> 1200 us there and 1171 -> 1145 us for
+// 21 k atoms of 16 slots, 56 candidates).  Two candidates a thread gave 530 us
+// there, but 48 for 35 us with one candidate.  Only the run without
+// allocations, whose workspace the caller sized, packs V to 24 bytes.
 constexpr int FORCE_LANES = 8;
 
+template <int VS>
 __global__ void __launch_bounds__(256)
     k_force(DevDb db, const double *__restrict__ V, double *__restrict__ aout, double *__restrict__ forces,
             double *__restrict__ errvec, int esize, double *__restrict__ lam) {
   const int c = blockIdx.y, N = db.natoms, l = threadIdx.x % FORCE_LANES;
   const int i0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) / FORCE_LANES), i = min(i0, N - 1);
   double *ao = aout + (size_t)c * AO_COUNT * N;
-  const double *Vc = V + (size_t)c * 3 * db.npairs;  // (x, y, z) per slot: one or two 32-byte sectors a read
+  const double *Vc = V + (size_t)c * VS * db.npairs;
   const int q1 = db.in_off[i + 1], cell = db.atom_cell[i], comp = min(l, 2);
   const double own = ao[(AO_AX + comp) * N + i], f0 = db.force0[3 * i + comp];
   double f[3] = {0.0, 0.0, 0.0};
 #pragma unroll 4
   for (int q = db.in_off[i] + l; q < q1; q += FORCE_LANES) {
-    const double *v = Vc + 3 * (int64_t)db.in_slot[q];
-    f[0] += v[0];
-    f[1] += v[1];
-    f[2] += v[2];
+    const double *v = Vc + VS * (int64_t)db.in_slot[q];
+    double x, y, z;
+    if (VS == 4) {
+      load_vec4(v, x, y, z);
+    } else {
+      x = v[0];
+      y = v[1];
+      z = v[2];
+    }
+    f[0] += x;
+    f[1] += y;
+    f[2] += z;
   }
 #pragma unroll
   for (int o = FORCE_LANES / 2; o > 0; o >>= 1)

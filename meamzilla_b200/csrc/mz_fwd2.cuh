@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(BLOCK_SLOTS, 4)
       const double ck = dF * fp * ip;
       const double Vx = ck * vx[c] + (double)ux * cu, Vy = ck * vy[c] + (double)uy * cu,
                    Vz = ck * vz[c] + (double)uz * cu;
-      double *Vc = Vout + (size_t)cand * 3 * Np + 3 * gs;  // (x, y, z) per slot
+      double *Vc = Vout + ((size_t)cand * Np + gs) * db.vs;  // (x, y, z) per slot
       Vc[0] = Vx;
       Vc[1] = Vy;
       Vc[2] = Vz;

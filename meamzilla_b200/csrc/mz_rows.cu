@@ -22,9 +22,12 @@ cudaError_t forward(const RowsForward &a) {
   // One group of atoms a warp and one candidate a CTA while that is less than
   // eight waves of CTAs (4 resident per SM); then up to four candidates, which
   // share the slots' loads, and up to eight groups, which share the tables.
+  // Without angular terms, where the loads are a larger part, up to eight
+  // candidates (18 k atoms of 42 slots, 128 candidates: 1408 -> 1329 us, 1383
+  // with sixteen; with angular terms 1171 -> 1221 us for 21 k atoms, 56).
   const int64_t groups = ((int64_t)a.db.natoms * LPA + 31) / 32;
   const int64_t ctas = (groups + ROWS_W - 1) / ROWS_W, wave = 4 * (int64_t)a.nsm;
-  int ncb = (int)std::min<int64_t>(std::min(a.ncand, 4), std::max<int64_t>(1, ctas * a.ncand / (8 * wave)));
+  int ncb = (int)std::min<int64_t>(std::min(a.ncand, a.meam ? 4 : 8), std::max<int64_t>(1, ctas * a.ncand / (8 * wave)));
   RowsLayout L = rows_forward_layout(a.pot, LPA, ncb);
   while (ncb > 1 && L.bytes > 48 * 1024) L = rows_forward_layout(a.pot, LPA, --ncb);  // four CTAs on an SM
   const int64_t ny = (a.ncand + ncb - 1) / ncb;

@@ -20,9 +20,9 @@
 // summed, and a lane's slots advance side by side (the FP64 pipe takes 1.8
 // instructions a clock from warps with four independent chains, 1.25 from
 // any number of warps with one).  Measured (k_atoms -> k_rows): 84 k atoms of
-// 41 slots, 1 candidate 581 -> 385 us (shared memory 71 %, FP64 52 %); 21 k
-// atoms of 16 slots, 56 candidates 2397 -> 1171 us; EAM, 18 k atoms of 42
-// slots, 128 candidates 4811 -> 1408 us.
+// 41 slots, 1 candidate 581 -> 379 us (shared memory 71 %, FP64 52 %); 21 k
+// atoms of 16 slots, 56 candidates 2397 -> 1145 us; EAM, 18 k atoms of 42
+// slots, 128 candidates 4811 -> 1200 us.
 #pragma once
 
 #include <type_traits>
@@ -55,7 +55,7 @@ struct RowsLayout {
 
 // per candidate: both piece tables as halves (c0, c1) and (c2, c3), the U
 // splines' knot table; then the geometry; then the warps' rows: (u_x, u_y),
-// (u_z, f) and per JMEAM term p; the neighbour types (GMEAM); reused for V
+// (u_z, f) and per JMEAM term p; the neighbour types (GMEAM)
 __host__ __device__ inline RowsLayout rows_layout(const DevPot &pot, int lpa, int spl, bool rows, int ncb) {
   RowsLayout L;
   L.npiece = pot.pow_stride / 4;
@@ -79,7 +79,7 @@ __host__ __device__ inline RowsLayout rows_layout(const DevPot &pot, int lpa, in
   b = (b + 15) & ~size_t(15);
   L.o_rows = b;
   L.row_bytes = rows ? (size_t)aw * L.rs * (2 * sizeof(double2) + sizeof(double) * pot.nj + (pot.gmeam ? sizeof(int) : 0))
-                     : (size_t)aw * L.rs * 3 * sizeof(double);
+                     : 0;
   L.row_bytes = (L.row_bytes + 15) & ~size_t(15);
   L.bytes = b + ROWS_W * L.row_bytes;
   return L;
@@ -291,7 +291,6 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
   double2 *rzf = reinterpret_cast<double2 *>(wrow) + (AW + sub) * L.rs;
   double *rp = reinterpret_cast<double *>(wrow + 2 * sizeof(double2) * AW * L.rs) + sub * L.rs;  // + m AW rs
   int *rt = reinterpret_cast<int *>(wrow + 2 * sizeof(double2) * AW * L.rs) + sub * L.rs;
-  double *rv = reinterpret_cast<double *>(wrow) + (size_t)sub * L.rs * 3;  // V of the atom's slots, after the rows
   const double2 *uxy = db.pair2, *uzr = uxy + Np, *irf = uzr + Np, *pr = irf + Np;
 
   const int ngroups = (N + AW - 1) / AW;
@@ -395,7 +394,7 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
               const int p = l + s * LPA, gs = lo + p;
               if (p >= n) continue;
               const double vx = v[s][0] * a->inv, vy = v[s][1] * a->inv, vz = v[s][2] * a->inv;
-              const double H = u[s][0] * vx + u[s][1] * vy + u[s][2] * vz;
+              const double H = fma(u[s][0], vx, fma(u[s][1], vy, u[s][2] * vz));
               const int2 m2 = db.pair_meta[gs];
               const int kp = m ? (int)db.pair_knot_p2[gs] : ((m2.x >> 24) & 0xff) - 1;
               if (kp >= 0) {
@@ -403,7 +402,7 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
                 double d;
                 const double pv = rows_piece(plo, phi, rg.poff / 4 + kp, db.pair_shift[(3 + m) * Np + gs], d);
                 const double pi = pv * irf[gs].x;
-                cd[s] += d * rg.invstep * S[s] - pi * H;
+                cd[s] += fma(d * rg.invstep, S[s], -(pi * H));
                 Vd[s][0] += pi * vx;
                 Vd[s][1] += pi * vy;
                 Vd[s][2] += pi * vz;
@@ -422,7 +421,8 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
         }
         pass(spl + (GM ? pot.s_g + ti * pot.npair : pot.s_g + ti), [](int, double f) { return f; });
       }
-      // ---- per slot: V = u (A + U' B) + U' C, with C left in v
+      // ---- per slot: V = u (A + U' B) + U' C, with C left in v.  Sums of products are written as fma, so that every
+      // instance of the kernel (with and without AUX) rounds alike.
       const double ginv = MEAM && !GM ? spl[pot.s_g + ti].inv : 1.0;
       double A[SPL], B[SPL], rho = 0.0, ep = e3;
 #pragma unroll
@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
         }
         if (MEAM) {
           const double vx = v[s][0] * ginv, vy = v[s][1] * ginv, vz = v[s][2] * ginv;
-          const double H = u[s][0] * vx + u[s][1] * vy + u[s][2] * vz;
+          const double H = fma(u[s][0], vx, fma(u[s][1], vy, u[s][2] * vz));
           const int kf = ((m2.x >> 16) & 0xff) - 1;
           const double2 c = irf[gs];  // 1 / r, shift of f
           double fi = 0.0;
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
             const double f = rows_piece(plo, phi, g.p0 + kf, c.y, d);
             rho += 0.5 * f * S[s];
             fi = f * c.x;
-            B[s] += d * g.inv * S[s] - fi * H;
+            B[s] += fma(d * g.inv, S[s], -(fi * H));
           }
           if (AUX) {
             double *ax = aux + (size_t)cand * pot.aux_rows * Np + gs;
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
 #pragma unroll
       for (int j = 0; j < 8; ++j) q[j] = 0.0;
       q[3] = ep;
-      if (MEAM) __syncwarp();  // the rows are read; V takes their place
+      double *Vc = Vout + 4 * ((size_t)cand * Np + lo);
 #pragma unroll
       for (int s = 0; s < SPL; ++s) {
         const int p = l + s * LPA;
@@ -508,9 +508,9 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
           V[k] = u[s][k] * cu;
           if (MEAM) V[k] = fma(dF, v[s][k], V[k]);
           if (JM) V[k] += Vd[s][k];
-          rv[3 * p + k] = V[k];
           q[k] += V[k];
         }
+        store_vec4(Vc + 4 * (int64_t)p, V[0], V[1], V[2]);
         const double r = KEEP ? rk[s] : uzr[lo + p].y, x = V[0] * r, y = V[1] * r, z = V[2] * r;
         q[4] -= u[s][0] * x;
         q[5] -= u[s][1] * y;
@@ -518,12 +518,6 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
         q[7] -= u[s][0] * y;
         s8 -= u[s][1] * z;
         s9 -= u[s][2] * x;
-      }
-      __syncwarp();
-      // the atom's V, contiguous: 24 bytes per slot
-      {
-        double *Vc = Vout + (size_t)cand * 3 * Np + 3 * (int64_t)lo;
-        for (int k = l; k < 3 * n; k += LPA) Vc[k] = rv[k];
       }
       rows_sums10<LPA>(q, s8, s9, l);
       if (live) {
@@ -537,7 +531,7 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
           ao[AO_RHO * N] = rho_raw;
         }
       }
-      __syncwarp();  // the next candidate or group reuses the rows
+      if (MEAM) __syncwarp();  // the next candidate or group reuses the rows
     }
   }
 }
