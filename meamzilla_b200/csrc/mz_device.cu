@@ -2,9 +2,11 @@
 // and the evaluator half of the C ABI (include/mz_b200.h).
 //
 // Launch sequence of one objective call (kernels in mz_fwd.cuh / mz_adj.cuh):
-//   k_prep    one thread per (candidate, spline): coefficients -> knot table,
-//             second derivatives by the reference's tridiagonal solve
+//   k_prep    one CTA per candidate: coefficients -> knot table, second
+//             derivatives by the reference's tridiagonal solve, as a matrix
 //             (Spline3Eq::refresh_basis, spline3eq.cpp:192-225).
+//   k_rows    (FP64, mz_rows.cuh) whole atoms per warp, up to four slots per
+//             lane; and in mixed precision, for long rows and spline5eq
 //   k_atoms   one CTA per (atom block, candidate), one thread per pair slot.
 //             The block's neighbour rows are staged in shared memory and
 //             triplets are enumerated implicitly as the other slots of the
@@ -22,6 +24,8 @@
 //             of squares + style punishments (pot_meam_spline.cpp:274-278,
 //             pot_eam_spline.cpp:211-218).
 // and for the gradient:
+//   k_rows_adj, k_rows_radial (FP64, mz_rows_adj.cuh): angular tables per lane,
+//                radial functions over slots sorted by knot interval; otherwise
 //   k_adj        persistent CTAs over atom blocks, one thread per slot
 //   k_grad_sum   the CTAs' partial sums
 //   k_grad_final punishment terms, transposed refresh.
@@ -475,6 +479,9 @@ bool rows_adj_prepare(mz_ctx *ctx) {
   auto &ra = ctx->radj;
   if (ra.ready) return true;
   if (ra.failed || !ctx->rows_ok || ctx->pot.nj > 0) return false;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  ck(cudaStreamIsCapturing(ctx->stream, &capture), "capture status");
+  if (capture != cudaStreamCaptureStatusNone) return false;  // a caller's capture allows no allocation
   const bool meam = style_meam(ctx->pot.style);
   const int N = ctx->natoms;
   const size_t C = ctx->cand_cap, Np = ctx->npairs;
