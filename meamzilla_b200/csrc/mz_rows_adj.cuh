@@ -114,7 +114,7 @@ __device__ __forceinline__ void radj_pass(const RadjRow &R, int nk, int l, const
     for (int s = 0; s < NS; ++s) T[s] = fma(Qx[s], u[s][0], fma(Qy[s], u[s][1], Qz[s] * u[s][2]));
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      const bool no = CL && (out[s] || !(c[s] < g[s].cut));
+      const bool no = out[s] || (CL && !(c[s] < g[s].cut));
       if (GM) T[s] *= g[s].inv;
       if (no) T[s] = 0.0;
       w[s] = f[s] * (no ? 0.0 : W[s]);
@@ -154,41 +154,28 @@ __device__ __forceinline__ void radj_pass(const RadjRow &R, int nk, int l, const
   double x[NS], y[NS], z[NS], W[NS], Qx[NS], Qy[NS], Qz[NS], qx[NS];
   bool out[NS];
   int tk[NS];
+#pragma unroll
+  for (int s0 = 0; s0 < NS; ++s0) {  // runs of LPA partners: the slot itself is none (see rows_pass)
+    const int len = min(nk - s0 * LPA, LPA);
 #pragma unroll 1
-  for (int k = 0; k < nk; ++k) {
-    const double2 a = R.uxy[k], c = R.uzw[k], d = R.qxy[k], e = R.qzx[k];
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      x[s] = a.x;
-      y[s] = a.y;
-      z[s] = c.x;
-      W[s] = c.y;
-      Qx[s] = d.x;
-      Qy[s] = d.y;
-      Qz[s] = e.x;
-      qx[s] = e.y;
-      out[s] = CL && k == l + s * LPA;
-      tk[s] = GM ? R.type[k] : 0;
-    }
-    step(x, y, z, W, Qx, Qy, Qz, qx, out, tk);
-  }
-  if (!CL) {  // the slot itself went through the loop: its term off again (see rows_pass)
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      const int k = l + s * LPA;
+    for (int i = 0; i < len; ++i) {
+      const int k = s0 * LPA + i;
       const double2 a = R.uxy[k], c = R.uzw[k], d = R.qxy[k], e = R.qzx[k];
-      x[s] = a.x;
-      y[s] = a.y;
-      z[s] = c.x;
-      W[s] = -c.y;
-      Qx[s] = -d.x;
-      Qy[s] = -d.y;
-      Qz[s] = -e.x;
-      qx[s] = -e.y;
-      out[s] = false;
-      tk[s] = GM ? R.type[k] : 0;
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        x[s] = a.x;
+        y[s] = a.y;
+        z[s] = c.x;
+        W[s] = c.y;
+        Qx[s] = d.x;
+        Qy[s] = d.y;
+        Qz[s] = e.x;
+        qx[s] = e.y;
+        out[s] = s == s0 && i == l;
+        tk[s] = GM ? R.type[k] : 0;
+      }
+      step(x, y, z, W, Qx, Qy, Qz, qx, out, tk);
     }
-    step(x, y, z, W, Qx, Qy, Qz, qx, out, tk);
   }
 }
 
