@@ -69,17 +69,19 @@ __global__ void __launch_bounds__(256)
   // With M, ypp = M (y, grad) (spline5eq: (ypp, yp4) = M (y, grad, grad2)): the
   // refreshes (Spline3Eq::refresh_basis, Spline5Eq::refresh_basis,
   // spline5eq.cpp:209-293) are linear, and M is solved once on the host.  A
-  // warp per spline, a lane per row.
+  // warp per spline, a lane per row.  A cubic's row r takes y - y_r, which its
+  // y'' depend on alone (the solve forms the same differences): the products
+  // of y itself would cancel, and their rounding grow with a constant in y.
   for (int s = warp; s < nsplines && M; s += T / 32) {
     const SplineGeom g = geom[s];
     const int n = g.n, nc = g.q5 ? n + 4 : n + 2;
     double *t = tab + g.toff;
     const double *g2 = t + 3 * n + 2;
     for (int r = lane; r < (g.q5 ? 2 * n : n); r += 32) {
-      const double *row = M + g.moff + (size_t)r * nc;
+      const double *row = M + g.moff + (size_t)r * nc, y0 = g.q5 ? 0.0 : t[r];
       double acc = 0.0;
 #pragma unroll 4
-      for (int q = 0; q < n; ++q) acc += row[q] * t[q];
+      for (int q = 0; q < n; ++q) acc += row[q] * (t[q] - y0);
       acc += row[n] * t[2 * n] + row[n + 1] * t[2 * n + 1];
       if (g.q5) acc += row[n + 2] * g2[0] + row[n + 3] * g2[1];
       if (r < n) t[n + r] = acc;
