@@ -279,6 +279,11 @@ mz_status mz_objective_device(mz_ctx *ctx, int ncand, const double *d_params, in
 mz_status mz_objective_grad_device(mz_ctx *ctx, int ncand, const double *d_params, int precision,
                                    double *d_obj, double *d_grad);
 mz_status mz_sync(mz_ctx *ctx);
+/* Sets the flag that a mixed-precision kernel sets when it gives up a bounded
+ * wait, as if one had: the next mz_sync or host-buffer call of a context that
+ * has run or captured such kernels fails with MZ_ERR_CUDA and clears it.  For
+ * tests of that path; no kernel has to fail for it. */
+mz_status mz_raise_device_flag(mz_ctx *ctx);
 /* The context's CUDA stream (a cudaStream_t), for callers that time or order
  * work against it. */
 void *mz_stream(mz_ctx *ctx);

@@ -118,6 +118,7 @@ _SIGS = {
     "mz_objective_device": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
     "mz_objective_grad_device": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
     "mz_sync": (C.c_int, [C.c_void_p]),
+    "mz_raise_device_flag": (C.c_int, [C.c_void_p]),
     "mz_stream": (C.c_void_p, [C.c_void_p]),
     "mz_gram_device": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int64, C.c_int, C.c_void_p, C.c_int64,
                                  C.c_int64, C.c_void_p]),

@@ -238,7 +238,9 @@ struct mz_ctx {
   bool io_tried = false, counted = false;
   double *c_params = nullptr, *c_obj = nullptr, *c_grad = nullptr;  // what the host calls' launches use
   int *c_flag = nullptr;
-  bool waits = false;  // kernels that can set the failure flag were launched since it was last read
+  // Kernels that can set the failure flag have been launched or captured: from
+  // then on every wait for the stream reads it (a caller may replay what it captured).
+  bool waits = false;
   double *d_gram = nullptr;  // partial sums of mz_gram_device, grown on demand
   size_t gram_cap = 0;       // doubles
   bool gram_ready[2] = {false, false};  // shared memory of k_gram_tile set (narrow, wide copies)
@@ -322,7 +324,6 @@ void release(mz_ctx *ctx) {
 // A kernel that gave up on a bounded wait sets the context's flag.
 void check_device_flag(mz_ctx *ctx) {
   if (!ctx->waits) return;
-  ctx->waits = false;
   int e = 0;
   ck(cudaMemcpy(&e, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost), "flag D2H");
   if (e) {
@@ -1401,6 +1402,9 @@ void run_host(mz_ctx *ctx, int ncand, const double *params, int precision, doubl
       ck(cudaMemcpyAsync(ctx->d_params, px, sizeof(double) * n * P, cudaMemcpyHostToDevice, ctx->stream), "params H2D");
     launch_objective(ctx, n, precision, errvec != nullptr, forces != nullptr, energy != nullptr, stress != nullptr,
                      grad != nullptr);
+    // a mixed call's sequence brings the flag itself; an FP64 call after mixed device calls fetches it too
+    if (ctx->waits && ctx->c_flag && !may_give_up(ctx, precision))
+      ck(cudaMemcpyAsync(ctx->c_flag, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "flag D2H");
     struct Out {
       double *host;
       const double *dev;
@@ -1433,9 +1437,8 @@ void run_host(mz_ctx *ctx, int ncand, const double *params, int precision, doubl
         std::memcpy(o.host, at, sizeof(double) * o.count);
         at += sizeof(double) * o.count;
       }
-    if (may_give_up(ctx, precision) && (!ctx->c_flag || *ctx->c_flag)) {
+    if (ctx->waits && (!ctx->c_flag || *ctx->c_flag)) {
       if (ctx->c_flag) *ctx->c_flag = 0;
-      ctx->waits = true;  // a replayed graph does not set it
       check_device_flag(ctx);
     }
   }
@@ -2016,6 +2019,16 @@ mz_status mz_sync(mz_ctx *ctx) {
     if (!ctx) throw Failure{MZ_ERR_ARG, "null context"};
     ck(cudaStreamSynchronize(ctx->stream), "sync");
     check_device_flag(ctx);
+  });
+}
+
+mz_status mz_raise_device_flag(mz_ctx *ctx) {
+  return guarded([&] {
+    if (!ctx) throw Failure{MZ_ERR_ARG, "null context"};
+    ck(cudaSetDevice(ctx->device), "cudaSetDevice");
+    const int e = 1;
+    ck(cudaMemcpyAsync(ctx->d_err, &e, sizeof(int), cudaMemcpyHostToDevice, ctx->stream), "flag H2D");
+    ck(cudaStreamSynchronize(ctx->stream), "flag H2D");
   });
 }
 
