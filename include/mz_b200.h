@@ -273,7 +273,13 @@ mz_status mz_densities(mz_ctx *ctx, const double *params, double *dens);
 
 /* Same as mz_objective with device pointers (params, obj, errvec, forces on
  * the device; any output may be null) enqueued on the context's stream; the
- * call returns before the work completes.  mz_sync waits for it. */
+ * call returns before the work completes.  mz_sync waits for it.  Both may be
+ * called inside a capture of that stream (a CUDA graph): they enqueue kernels
+ * only.  What a context prepares at the first call of a precision, with or
+ * without the gradient, outside a capture (launch variants, the FP64
+ * gradient's sorted lists, the moment path) is not made inside one: a capture
+ * before that call runs the variants that need no preparation, whose sums
+ * round differently and which may be slower. */
 mz_status mz_objective_device(mz_ctx *ctx, int ncand, const double *d_params, int precision,
                               double *d_obj, double *d_errvec, double *d_forces);
 mz_status mz_objective_grad_device(mz_ctx *ctx, int ncand, const double *d_params, int precision,

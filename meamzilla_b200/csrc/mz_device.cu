@@ -480,9 +480,6 @@ bool rows_adj_prepare(mz_ctx *ctx) {
   auto &ra = ctx->radj;
   if (ra.ready) return true;
   if (ra.failed || !ctx->rows_ok || ctx->pot.nj > 0) return false;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  ck(cudaStreamIsCapturing(ctx->stream, &capture), "capture status");
-  if (capture != cudaStreamCaptureStatusNone) return false;  // a caller's capture allows no allocation
   const bool meam = style_meam(ctx->pot.style);
   const int N = ctx->natoms;
   const size_t C = ctx->cand_cap, Np = ctx->npairs;
@@ -1185,31 +1182,44 @@ double trial(mz_ctx *ctx, int n, const double *d_params, int precision, bool gra
 // Picks, once per (precision, gradient), the forward's atoms per block, then
 // the adjoint's atoms per block and persistent CTAs, by timing each on the
 // caller's own candidates; MZ_TUNE=0 keeps the first variant of each.
+// Inside a caller's capture of the stream nothing can be timed or allocated:
+// a call that finds no choice made runs the first variant (FP64 gradients the
+// block kernels, mixed calls the row kernels), and the choice is left open.
 void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, bool grad) {
-  if (precision == MZ_FP64 && grad) rows_adj_prepare(ctx);
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  ck(cudaStreamIsCapturing(ctx->stream, &status), "capture status");
+  const bool capturing = status != cudaStreamCaptureStatusNone;
+  if (precision == MZ_FP64 && grad && !capturing) rows_adj_prepare(ctx);
   mz_ctx::Tune &t = ctx->tune[precision][grad ? 1 : 0];
   if (!t.done) {
     const std::vector<int64_t> key = {ctx->device,     ctx->natoms,    ctx->npairs, ctx->ncells, ctx->pot.style,
                                       ctx->pot.ntypes, ctx->P,         precision,   grad,        ctx->q5,
                                       ctx->autotune,   ctx->nblk[0],   ctx->nadjblk[0], ctx->fm_mode};
     bool cached = false;
+    mz_ctx::Tune best;
     {
       std::lock_guard<std::mutex> lk(g_tune_mu);
       auto it = g_tune_cache.find(key);
       if (it != g_tune_cache.end()) {
-        t = it->second;
+        best = it->second;
         cached = true;
       }
     }
-    if (cached && t.fm && !fm_prepare(ctx)) t.fm = false;
     if (!cached) {
-      mz_ctx::Tune best;
       best.ctas = adj_ctas_for(ctx, 0, ctx->adj_per_sm);
       if (ctx->autotune == 2 && precision == MZ_MIXED && ctx->nc2_ok) {
         best.nc = 2;
         best.adj_nc = 2;
         best.ctas = adj_ctas_for(ctx, 0, ctx->adj2_per_sm);
       }
+    }
+    if (capturing) {
+      best.fm = ctx->fm.ready && (best.fm || (precision == MZ_MIXED && ctx->fm_mode == 2));
+      apply_variant(ctx, best);
+      return;
+    }
+    if (cached && best.fm && !fm_prepare(ctx)) best.fm = false;
+    if (!cached) {
       // the FP64 row kernels have no variants to time
       bool fixed = precision == MZ_FP64 && ctx->rows_ok && (!grad || ctx->radj.ready);
       // Nor are the mixed row kernels' worth timing where the moment path beats
@@ -1295,10 +1305,10 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
         }
       }
       best.done = true;
-      t = best;
       std::lock_guard<std::mutex> lk(g_tune_mu);
       g_tune_cache.emplace(key, best);
     }
+    t = best;
     t.done = true;
   }
   apply_variant(ctx, t);
