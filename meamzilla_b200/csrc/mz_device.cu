@@ -444,9 +444,22 @@ void launch_adj(mz_ctx *ctx, int n, size_t smem) {
                                                             ctx->d_partial, ctx->d_wglob);
 }
 
-template <class K>
-void smem_attr(K kernel, size_t bytes) {
-  ck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attribute");
+// Lets a kernel take `bytes` of dynamic shared memory.  The limit belongs to
+// the kernel on the device, not to a context: every context sets the largest
+// one, so that none lowers what another's launches need.
+void smem_attr(const void *kernel, size_t bytes) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes fa{};
+  ck(cudaGetDevice(&dev), "device");
+  ck(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "attribute");
+  ck(cudaFuncGetAttributes(&fa, kernel), "kernel attributes");
+  const size_t most = (size_t)optin - fa.sharedSizeBytes;
+  ck(bytes <= most ? cudaSuccess : cudaErrorInvalidValue, "smem attribute");
+  ck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most), "smem attribute");
+}
+template <class... A>
+void smem_attr(void (*kernel)(A...), size_t bytes) {
+  smem_attr(reinterpret_cast<const void *>(kernel), bytes);
 }
 
 void launch_grad_sum(mz_ctx *ctx, int n, const GradSums &g) {
@@ -490,6 +503,7 @@ bool rows_adj_prepare(mz_ctx *ctx) {
     a.pot = ctx->pot;
     a.meam = meam;
     a.max_row = ctx->max_row;
+    a.smem_block = ctx->smem_optin;
     RadialPlan &R = a.radial;
     R = RadialPlan{};
     R.nfun = meam ? 3 : ctx->pot.pair ? 1 : 2;
@@ -871,8 +885,9 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
     Bracket b(ctx, MZ_K_ATOMS);
     const size_t sa = ctx->smem_atoms[mixed ? 1 : 0];
     if (!mixed && ctx->rows_ok) {
-      RowsForward a{ctx->db,     ctx->pot,    meam,         ctx->max_row, n, ctx->nsm, ctx->d_geom, ctx->d_tabs,
-                    ctx->d_ptabs, ctx->d_V,   ctx->d_aout,  grad && meam ? ctx->d_aux : nullptr, st};
+      RowsForward a{ctx->db,     ctx->pot,     meam,       ctx->max_row, n,
+                    ctx->nsm,    ctx->smem_optin, ctx->d_geom, ctx->d_tabs, ctx->d_ptabs,
+                    ctx->d_V,    ctx->d_aout,  grad && meam ? ctx->d_aux : nullptr, st};
       ck(rows_forward(a), "k_rows launch");
     } else if (meam && mixed && ctx->tc_ok) {
       ctx->waits = true;
@@ -1851,8 +1866,7 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     if (ctx->adj_fits[1]) smem_attr(k_adj<true, float, true, false, true>, ctx->smem_adj[1]);
     if (ctx->adj_fits[0]) smem_attr(k_adj<true, double, false, true, true>, ctx->smem_adj[0]);
     if (ctx->adj_fits[1]) smem_attr(k_adj<true, float, false, true, true>, ctx->smem_adj[1]);
-    if (2 * sizeof(double) * stride > 48 * 1024 && 2 * sizeof(double) * stride <= (size_t)smem_max)
-      smem_attr(k_grad_final, 2 * sizeof(double) * stride);
+    if (2 * sizeof(double) * stride <= (size_t)smem_max) smem_attr(k_grad_final, 2 * sizeof(double) * stride);
     int nsm = 0, per_sm = 0;
     ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device), "attribute");
     if (ctx->adj_fits[1])
@@ -2363,9 +2377,7 @@ extern "C" mz_status mz_objective_noalloc(const mz_db *dbh, const mz_pot *poth, 
       base_ptr = static_cast<unsigned char *>(g_noalloc_addr[set->device]);
     }
     const size_t sa = atoms_smem_bytes<double>(ns, pstride);
-    ck(cudaFuncSetAttribute(meam ? (const void *)k_atoms<true, double, false> : (const void *)k_atoms<false, double, false>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sa),
-       "smem attribute");
+    smem_attr(meam ? (const void *)k_atoms<true, double, false> : (const void *)k_atoms<false, double, false>, sa);
     auto put = [&](size_t at, const void *src, size_t bytes) {
       if (bytes) ck(cudaMemcpy(base_ptr + at, src, bytes, cudaMemcpyHostToDevice), "cudaMemcpy H2D");
     };

@@ -32,8 +32,8 @@ cudaError_t forward(const RowsForward &a) {
   while (ncb > 1 && L.bytes > 48 * 1024) L = rows_forward_layout(a.pot, LPA, --ncb);  // four CTAs on an SM
   const int64_t ny = (a.ncand + ncb - 1) / ncb;
   const int64_t it = std::min<int64_t>(8, std::max<int64_t>(1, ctas * ny / (8 * wave)));
-  if (L.bytes > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes);
+  if (L.bytes > 48 * 1024) {  // the limit is the kernel's, shared by all contexts: always the largest
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smem_block);
     if (e != cudaSuccess) return e;
   }
   k<<<dim3((unsigned)((ctas + it - 1) / it), (unsigned)ny), 32 * ROWS_W, L.bytes, a.stream>>>(

@@ -13,6 +13,7 @@ struct RowsForward {
   bool meam;          // a style with angular terms
   int max_row;        // longest neighbour row
   int ncand, nsm;
+  int smem_block;     // most shared memory a block may opt into
   const SplineGeom *geom;
   const double *tabs, *ptabs;  // knot tables, evaluation tables of the candidates
   double *V, *aout;            // reaction vectors, per-atom sums
@@ -43,7 +44,7 @@ struct RowsAdjoint {
   DevDb db;
   DevPot pot;
   bool meam;
-  int max_row, ncand;
+  int max_row, ncand, smem_block;
   RadialPlan radial;
   const int4 *desc;    // groups of atoms, see k_rows_adj
   int ngroups;

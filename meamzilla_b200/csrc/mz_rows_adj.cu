@@ -56,7 +56,8 @@ cudaError_t rows_sort(const DevDb &db, const DevPot &pot, const RadialPlan &R, c
 cudaError_t rows_adjoint(const RowsAdjoint &a) {
   const RadjLayout L = radj_layout(a.pot, rows_lpa(a.max_row), a.meam, a.warps);
   AdjKernel k = kernel(a);
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes);
+  // the limit is the kernel's, shared by all contexts: always the largest
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smem_block);
   if (e != cudaSuccess) return e;
   k<<<dim3(a.ctas, a.ncand), 32 * L.warps, L.bytes, a.stream>>>(a.db, a.pot, L, a.desc, a.ngroups, a.geom, a.tabs,
                                                                a.ptabs, a.aout, a.aux, a.lam, a.seeds, a.W1, a.part);
