@@ -281,6 +281,7 @@ T *dupload(mz_ctx *ctx, const T *h, size_t n) {
 
 template <class F>
 mz_status guarded(F &&f) {
+  cudaGetLastError();  // an error that another call of this thread left is not this one's
   try {
     f();
     set_error("");

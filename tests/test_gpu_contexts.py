@@ -79,3 +79,17 @@ def test_threads_with_contexts_of_their_own():
     assert not errors, errors
     for ev, x, obj, grad, o, g in work:
         assert torch.equal(obj, o) and torch.equal(grad, g)
+
+
+def test_an_error_left_by_another_call():
+    """The CUDA runtime keeps a failed call's code until somebody asks for it:
+    an entry point does not take one that was there before it as its own."""
+    from meamzilla_b200.potential import MZ_FP64, Evaluator
+    ev, X = _evaluator("eam/spline", 1, 10, 8, 2)
+    value = ev.objective(X, MZ_FP64)
+    cudart = C.CDLL("libcudart.so.12")
+    assert cudart.cudaSetDevice(99) != 0
+    other = Evaluator(ev.db, ev.pot, 1.0, 1.0, 0, max_candidates=1)
+    assert np.array_equal(other.objective(X, MZ_FP64), value)
+    assert cudart.cudaSetDevice(99) != 0
+    assert np.array_equal(ev.objective(X, MZ_FP64), value)
