@@ -272,10 +272,13 @@ T *dalloc(mz_ctx *ctx, size_t n) {
   return static_cast<T *>(p);
 }
 
+// Copies go on the context's own stream, in front of the kernels that read
+// them: it does not wait for the default stream, and a copy from pageable
+// memory there may return while its last part is still on the way.
 template <class T>
 T *dupload(mz_ctx *ctx, const T *h, size_t n) {
   T *d = dalloc<T>(ctx, n);
-  if (n) ck(cudaMemcpy(d, h, n * sizeof(T), cudaMemcpyHostToDevice), "cudaMemcpy H2D");
+  if (n) ck(cudaMemcpyAsync(d, h, n * sizeof(T), cudaMemcpyHostToDevice, ctx->stream), "copy H2D");
   return d;
 }
 
@@ -328,7 +331,7 @@ void check_device_flag(mz_ctx *ctx) {
   int e = 0;
   ck(cudaMemcpy(&e, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost), "flag D2H");
   if (e) {
-    ck(cudaMemset(ctx->d_err, 0, sizeof(int)), "flag reset");
+    ck(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream), "flag reset");
     throw Failure{MZ_ERR_CUDA, "a tensor-core completion wait timed out on the device"};
   }
 }
@@ -1117,8 +1120,9 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Device buffers that live for one block of code.
+// Device buffers that live for one block of code, filled on one stream.
 struct Scratch {
+  cudaStream_t st;
   std::vector<void *> p;
   template <class T>
   const T *upload(const T *h, size_t n) {
@@ -1128,7 +1132,7 @@ struct Scratch {
       throw Failure{MZ_ERR_NOMEM, std::string("device allocation of ") + std::to_string(n * sizeof(T)) +
                                       " bytes failed: " + cudaGetErrorString(e)};
     p.push_back(d);
-    if (n) ck(cudaMemcpy(d, h, n * sizeof(T), cudaMemcpyHostToDevice), "cudaMemcpy H2D");
+    if (n) ck(cudaMemcpyAsync(d, h, n * sizeof(T), cudaMemcpyHostToDevice, st), "copy H2D");
     return static_cast<const T *>(d);
   }
   ~Scratch() {
@@ -1618,7 +1622,7 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
       pl.meta = dalloc<int2>(ctx, Np);
     }
     {
-      Scratch raw;
+      Scratch raw{ctx->stream, {}};
       const double *h_u = raw.upload(db.pair_u.data(), 3 * Np), *h_shift = raw.upload(db.pair_shift.data(), nf * Np);
       const signed char *h_knot = raw.upload(reinterpret_cast<const signed char *>(db.pair_knot.data()), nf * Np);
       if (Np > 0)
@@ -1955,11 +1959,11 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     ctx->d_grad = dalloc<double>(ctx, C * ctx->P);
     ctx->d_gsum = dalloc<double>(ctx, C * stride);
     ctx->d_count = dalloc<int>(ctx, C);
-    ck(cudaMemset(ctx->d_count, 0, sizeof(int) * C), "count init");
+    ck(cudaMemsetAsync(ctx->d_count, 0, sizeof(int) * C, ctx->stream), "count init");
     ctx->d_ptabf = dalloc<float>(ctx, C * ctx->pstride);
     ctx->d_wtab = meam ? dalloc<float>(ctx, C * pot.ntypes * (2 * TC_NB - 1)) : nullptr;
     ctx->d_err = dalloc<int>(ctx, 1);
-    ck(cudaMemset(ctx->d_err, 0, sizeof(int)), "flag init");
+    ck(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream), "flag init");
     *out = ctx;
   });
   if (st != MZ_OK && ctx) {

@@ -93,3 +93,15 @@ def test_an_error_left_by_another_call():
     assert np.array_equal(other.objective(X, MZ_FP64), value)
     assert cudart.cudaSetDevice(99) != 0
     assert np.array_equal(ev.objective(X, MZ_FP64), value)
+
+
+def test_first_call_right_after_creation():
+    """What a context is made of is there when its first kernels run: sixty
+    contexts of small arrays, each evaluated at once, give one value."""
+    from meamzilla_b200.potential import MZ_FP64, Evaluator
+    ev, X = _evaluator("meam/spline", 2, 10, 8, 2)
+    obj, grad = ev.objective_grad(X, MZ_FP64)
+    for _ in range(60):
+        other = Evaluator(ev.db, ev.pot, 1.0, 1.0, 0, max_candidates=1)
+        o, g = other.objective_grad(X, MZ_FP64)
+        assert np.array_equal(o, obj) and np.array_equal(g, grad)
