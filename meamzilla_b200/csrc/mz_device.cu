@@ -36,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -661,7 +662,7 @@ bool fm_prepare(mz_ctx *ctx) {
   };
   Need need[] = {
       {ctx->d_aux, sizeof(double) * C * aux_rows * Np, 2 * sizeof(float) * G * Q * 3 * CG},  // Y, Yb
-      {ctx->d_V, sizeof(double) * C * 4 * Np, sizeof(double) * Cp * Np * 3},                   // V
+      {ctx->d_V, sizeof(double) * C * ctx->db.vs * Np, sizeof(double) * Cp * Np * 3},          // V
       {ctx->d_aout, sizeof(double) * C * AO_COUNT * N, sizeof(double) * Cp * AO_COUNT * N},    // aoutF
       {ctx->d_lam, sizeof(double) * C * 3 * N, sizeof(float) * Cp * 3 * N},                    // lamf
       {ctx->d_seeds, sizeof(double) * C * CS_COUNT * NC, sizeof(double) * Cp * CS_COUNT * NC}, // seedF
@@ -917,7 +918,8 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
   if (!d_obj) return;
   {
     Bracket b(ctx, MZ_K_GATHER);
-    k_force<4><<<dim3((unsigned)(((int64_t)ctx->natoms * FORCE_LANES + 255) / 256), n), 256, 0, st>>>(
+    auto force = ctx->db.vs == 4 ? k_force<4> : k_force<3>;
+    force<<<dim3((unsigned)(((int64_t)ctx->natoms * FORCE_LANES + 255) / 256), n), 256, 0, st>>>(
         ctx->db, ctx->d_V, ctx->d_aout, d_forces, d_errvec, ctx->esize, grad ? ctx->d_lam : nullptr);
     ck(cudaGetLastError(), "k_force launch");
   }
@@ -1079,7 +1081,7 @@ int packed_knots(const Db &db, int64_t s) {
 }
 
 // The per-slot arrays of DevDb from the database's own (unit vectors (x, y, z)
-// per slot, shifts and knots [Np][nf]).
+// per slot, shifts and knots [Np][nf]; u, shift and knot here start at slot s0).
 struct PairLayout {
   double *u[3], *shift;
   float *f[4], *shiftf;  // u_x, u_y, u_z, r
@@ -1089,12 +1091,13 @@ struct PairLayout {
   int2 *meta;
 };
 __global__ void __launch_bounds__(256)
-    k_pair_layout(int64_t Np, int nf, const double *__restrict__ r, const double *__restrict__ u,
+    k_pair_layout(int64_t Np, int64_t s0, int n, int nf, const double *__restrict__ r, const double *__restrict__ u,
                   const double *__restrict__ shift, const signed char *__restrict__ knot, const int *__restrict__ nbr,
                   const int *__restrict__ type, PairLayout o) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= Np) return;
-  const double x = u[3 * s], y = u[3 * s + 1], z = u[3 * s + 2], rr = r[s];
+  const int q0 = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q0 >= n) return;
+  const int64_t s = s0 + q0;
+  const double x = u[3 * q0], y = u[3 * q0 + 1], z = u[3 * q0 + 2], rr = r[s];
   o.u[0][s] = x;
   o.u[1][s] = y;
   o.u[2][s] = z;
@@ -1102,20 +1105,20 @@ __global__ void __launch_bounds__(256)
   o.f[1][s] = (float)y;
   o.f[2][s] = (float)z;
   o.f[3][s] = (float)rr;
+  shift += (int64_t)nf * q0;
   for (int q = 0; q < nf; ++q) {
-    const double b = shift[nf * s + q];
-    o.shift[q * Np + s] = b;
-    o.shiftf[q * Np + s] = (float)b;
+    o.shift[q * Np + s] = shift[q];
+    o.shiftf[q * Np + s] = (float)shift[q];
   }
-  const signed char *k = knot + nf * s;
+  const signed char *k = knot + (int64_t)nf * q0;
   const int kn = (k[0] + 1) | ((k[1] + 1) << 8) | ((k[2] + 1) << 16) | (nf > 3 ? (k[3] + 1) << 24 : 0);
   o.knot[s] = kn;
   if (o.knot_p2) o.knot_p2[s] = k[4];
   if (o.pair2) {
     o.pair2[s] = make_double2(x, y);
     o.pair2[Np + s] = make_double2(z, rr);
-    o.pair2[2 * Np + s] = make_double2(1.0 / rr, shift[nf * s + 2]);
-    o.pair2[3 * Np + s] = make_double2(shift[nf * s], shift[nf * s + 1]);
+    o.pair2[2 * Np + s] = make_double2(1.0 / rr, shift[2]);
+    o.pair2[3 * Np + s] = make_double2(shift[0], shift[1]);
     o.meta[s] = make_int2(kn, type[nbr[s]]);
   }
 }
@@ -1125,15 +1128,18 @@ struct Scratch {
   cudaStream_t st;
   std::vector<void *> p;
   template <class T>
-  const T *upload(const T *h, size_t n) {
+  T *get(size_t n) {
     void *d = nullptr;
     const cudaError_t e = cudaMalloc(&d, std::max<size_t>(1, n) * sizeof(T));
     if (e != cudaSuccess)
       throw Failure{MZ_ERR_NOMEM, std::string("device allocation of ") + std::to_string(n * sizeof(T)) +
                                       " bytes failed: " + cudaGetErrorString(e)};
     p.push_back(d);
+    return static_cast<T *>(d);
+  }
+  template <class T>
+  void put(T *d, const T *h, size_t n) {
     if (n) ck(cudaMemcpyAsync(d, h, n * sizeof(T), cudaMemcpyHostToDevice, st), "copy H2D");
-    return static_cast<const T *>(d);
   }
   ~Scratch() {
     for (void *d : p) cudaFree(d);
@@ -1584,7 +1590,6 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     d.ncells = db.ncells;
     d.natoms = N;
     d.npairs = Np;
-    d.vs = 4;
     d.cell_atom0 = dupload(ctx, db.cell_atom0.data(), db.cell_atom0.size());
     d.cell_vol = dupload(ctx, db.cell_vol.data(), db.cell_vol.size());
     d.cell_w = dupload(ctx, db.cell_weight.data(), db.cell_weight.size());
@@ -1617,18 +1622,39 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     pl.shiftf = dalloc<float>(ctx, nf * Np);
     pl.knot = dalloc<int>(ctx, Np);
     pl.knot_p2 = nf > 4 ? dalloc<signed char>(ctx, Np) : nullptr;
+    // a candidate's bytes in the work buffers below, with V of vs doubles per slot
+    const auto cand_bytes = [&](int vs) {
+      return sizeof(double) * ((size_t)(vs + (meam ? dp.aux_rows : 0)) * Np + (size_t)(AO_COUNT + 3 + 3) * N +
+                               (size_t)ctx->esize + (size_t)(8 + 1 + CS_COUNT) * db.ncells);
+    };
+    // The FP64 row kernels' copies (72 bytes a slot), unless memory is short:
+    // where the asked candidates do not fit beside them, they may take a 16th of it.
+    size_t copies = 0;
     if (!ctx->q5 && rows_lpa(db.max_row) > 0) {
-      pl.pair2 = dalloc<double2>(ctx, 4 * Np);
-      pl.meta = dalloc<int2>(ctx, Np);
+      size_t freeb = 0, totalb = 0;
+      ck(cudaMemGetInfo(&freeb, &totalb), "cudaMemGetInfo");
+      const size_t want = Np * (4 * sizeof(double2) + sizeof(int2));
+      if (want <= freeb / 16 || want + (double)ctx->max_cand * cand_bytes(4) <= 0.6 * (double)freeb) {
+        pl.pair2 = dalloc<double2>(ctx, 4 * Np);
+        pl.meta = dalloc<int2>(ctx, Np);
+        copies = want;
+      }
     }
     {
+      // through staging buffers of a few million slots: the work buffers may need the rest
       Scratch raw{ctx->stream, {}};
-      const double *h_u = raw.upload(db.pair_u.data(), 3 * Np), *h_shift = raw.upload(db.pair_shift.data(), nf * Np);
-      const signed char *h_knot = raw.upload(reinterpret_cast<const signed char *>(db.pair_knot.data()), nf * Np);
-      if (Np > 0)
-        k_pair_layout<<<(unsigned)((Np + 255) / 256), 256, 0, ctx->stream>>>(Np, nf, d.pair_r, h_u, h_shift, h_knot,
-                                                                            d.pair_nbr, d.atom_type, pl);
-      ck(cudaGetLastError(), "k_pair_layout launch");
+      const int64_t most = std::min<int64_t>(Np, 4 << 20);
+      double *h_u = raw.get<double>(3 * most), *h_shift = raw.get<double>(nf * most);
+      signed char *h_knot = raw.get<signed char>(nf * most);
+      for (int64_t s0 = 0; s0 < Np; s0 += most) {
+        const int n = (int)std::min(most, Np - s0);
+        raw.put(h_u, db.pair_u.data() + 3 * s0, 3 * (size_t)n);
+        raw.put(h_shift, db.pair_shift.data() + nf * s0, nf * (size_t)n);
+        raw.put(h_knot, reinterpret_cast<const signed char *>(db.pair_knot.data()) + nf * s0, nf * (size_t)n);
+        k_pair_layout<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(Np, s0, n, nf, d.pair_r, h_u, h_shift,
+                                                                           h_knot, d.pair_nbr, d.atom_type, pl);
+        ck(cudaGetLastError(), "k_pair_layout launch");
+      }
       ck(cudaStreamSynchronize(ctx->stream), "pair layout");
     }
     d.pair_ux = pl.u[0];
@@ -1810,7 +1836,7 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     ck(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device), "attribute");
     ctx->smem_optin = smem_max;
     ctx->max_row = db.max_row;
-    ctx->rows_ok = !ctx->q5 && rows_lpa(db.max_row) > 0 &&
+    ctx->rows_ok = d.pair2 != nullptr &&
                    rows_forward_bytes(dp, rows_lpa(db.max_row)) <= (size_t)smem_max;
     if (ctx->smem_atoms[0] > (size_t)smem_max)
       throw Failure{MZ_ERR_RANGE, "potential too large for the kernels' shared-memory tables"};
@@ -1928,20 +1954,20 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     // ---- work buffers: candidates per launch bounded by device memory
     size_t freeb = 0, totalb = 0;
     ck(cudaMemGetInfo(&freeb, &totalb), "cudaMemGetInfo");
-    const size_t per_cand =
-        sizeof(double) * ((size_t)(4 + (meam ? dp.aux_rows : 0)) * Np + (size_t)(AO_COUNT + 3 + 3) * N +
-                          (size_t)ctx->esize + (size_t)(8 + 1 + CS_COUNT) * db.ncells + 2 * (size_t)stride + ctx->pstride +
-                          (size_t)ctx->adj_ctas_max * stride * (1 + ADJ_WARPS) + (size_t)2049 * stride +
-                          2 * (size_t)ctx->P + 1) +
-        sizeof(int);
-    const size_t budget = (size_t)(0.6 * (double)freeb);
-    const int cap = (int)std::max<size_t>(1, budget / std::max<size_t>(per_cand, 1));
+    // V as 32-byte records where the asked candidates fit with them, else packed:
+    // neither the records nor the row kernels' copies make a launch hold fewer.
+    const size_t tables = sizeof(double) * (2 * (size_t)stride + ctx->pstride +
+                                            (size_t)ctx->adj_ctas_max * stride * (1 + ADJ_WARPS) + (size_t)2048 * stride +
+                                            2 * (size_t)ctx->P + 1);
+    const size_t budget = (size_t)(0.6 * (double)(freeb + copies));
+    const int cap = (int)std::min<size_t>(INT_MAX, std::max<size_t>(1, budget / (cand_bytes(3) + tables)));
     ctx->cand_cap = std::min(ctx->max_cand, cap);
+    d.vs = ctx->cand_cap * (cand_bytes(4) + tables) <= budget ? 4 : 3;
     const size_t C = ctx->cand_cap;
     ctx->d_params = dalloc<double>(ctx, C * ctx->P);
     ctx->d_tabs = dalloc<double>(ctx, C * stride);
     ctx->d_ptabs = dalloc<double>(ctx, C * ctx->pstride);
-    ctx->d_V = dalloc<double>(ctx, C * 4 * Np);
+    ctx->d_V = dalloc<double>(ctx, C * d.vs * Np);
     ctx->d_aout = dalloc<double>(ctx, C * AO_COUNT * N);
     ctx->d_forces = dalloc<double>(ctx, C * 3 * N);
     ctx->d_cellobj = dalloc<double>(ctx, C * db.ncells);

@@ -647,8 +647,9 @@ __global__ void __launch_bounds__(BLOCK_SLOTS, JM ? 2 : sizeof(R) == 4 ? 4 : 3)
 // atoms of 42 slots, 128 candidates: 592 -> 558 us, 5.2 TB/s; k_rows, which
 // writes them without staging, 1408 -> 1200 us there and 1171 -> 1145 us for
 // 21 k atoms of 16 slots, 56 candidates).  Two candidates a thread gave 530 us
-// there, but 48 for 35 us with one candidate.  Only the run without
-// allocations, whose workspace the caller sized, packs V to 24 bytes.
+// there, but 48 for 35 us with one candidate.  V is packed to 24 bytes where
+// records would make a launch hold fewer candidates than were asked for, and
+// in the run without allocations, whose workspace the caller sized.
 constexpr int FORCE_LANES = 8;
 
 template <int VS>

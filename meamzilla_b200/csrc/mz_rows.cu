@@ -16,9 +16,9 @@ RowsLayout rows_forward_layout(const DevPot &pot, int lpa, int ncb) {
   return rows_layout(pot, lpa, 4, pot.s_g > 0, ncb);
 }
 
-template <bool MEAM, bool AUX, bool GM, bool JM, int LPA>
+template <bool MEAM, bool AUX, bool GM, bool JM, int LPA, int VS = 0>
 cudaError_t forward(const RowsForward &a) {
-  auto k = k_rows<MEAM, AUX, GM, JM, LPA, 4>;
+  auto k = k_rows<MEAM, AUX, GM, JM, LPA, 4, VS>;
   // One group of atoms a warp and one candidate a CTA while that is less than
   // eight waves of CTAs (4 resident per SM); then up to four candidates, which
   // share the slots' loads, and up to eight groups, which share the tables.
@@ -43,7 +43,8 @@ cudaError_t forward(const RowsForward &a) {
 
 template <int LPA>
 cudaError_t forward_lpa(const RowsForward &a) {
-  if (!a.meam) return forward<false, false, false, false, LPA>(a);
+  if (!a.meam)
+    return a.db.vs == 4 ? forward<false, false, false, false, LPA, 4>(a) : forward<false, false, false, false, LPA, 3>(a);
   if (a.pot.nj > 0)
     return a.aux ? forward<true, true, false, true, LPA>(a) : forward<true, false, false, true, LPA>(a);
   if (a.pot.gmeam)
