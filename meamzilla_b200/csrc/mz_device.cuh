@@ -15,6 +15,17 @@ __device__ __forceinline__ void store_vec4(double *p, double x, double y, double
   asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" : : "l"(p), "d"(x), "d"(y), "d"(z), "d"(0.0) : "memory");
 }
 
+// a slot's pair force in its record (vs = 4) or packed (3)
+__device__ __forceinline__ void store_vec(double *p, int vs, double x, double y, double z) {
+  if (vs == 4) {
+    store_vec4(p, x, y, z);
+  } else {
+    p[0] = x;
+    p[1] = y;
+    p[2] = z;
+  }
+}
+
 constexpr int MAX_SPLINES = 64;     // splines in one potential (8 types MEAM: 36+8+8+36+8)
 constexpr int BLOCK_SLOTS = 256;    // pair slots (threads) of one atom block
 constexpr int BLOCK_ATOMS = 64;     // atoms of one atom block

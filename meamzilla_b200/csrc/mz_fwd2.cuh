@@ -258,9 +258,7 @@ __global__ void __launch_bounds__(BLOCK_SLOTS, 4)
       const double Vx = ck * vx[c] + (double)ux * cu, Vy = ck * vy[c] + (double)uy * cu,
                    Vz = ck * vz[c] + (double)uz * cu;
       double *Vc = Vout + ((size_t)cand * Np + gs) * db.vs;  // (x, y, z) per slot
-      Vc[0] = Vx;
-      Vc[1] = Vy;
-      Vc[2] = Vz;
+      store_vec(Vc, db.vs, Vx, Vy, Vz);
       const double r = db.pair_r[gs];
       const double dx = db.pair_ux[gs], dy = db.pair_uy[gs], dz = db.pair_uz[gs];
       red[0 * BLOCK_SLOTS + tid] = Vx;

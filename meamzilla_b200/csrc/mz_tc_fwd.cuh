@@ -387,9 +387,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const double ck = dF * (double)f * ip;
         const double Vx = ux * cu + ck * vx, Vy = uy * cu + ck * vy, Vz = uz * cu + ck * vz;
         double *Vc = Vout + ((size_t)cand * Np + s) * db.vs;  // (x, y, z) per slot
-        Vc[0] = Vx;
-        Vc[1] = Vy;
-        Vc[2] = Vz;
+        store_vec(Vc, db.vs, Vx, Vy, Vz);
         if (AUX) {
           double *ax = aux + (size_t)cand * AUX_COUNT * Np;
           ax[AUX_G * Np + s] = G;
