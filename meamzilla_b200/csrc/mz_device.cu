@@ -1956,13 +1956,15 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
     ck(cudaMemGetInfo(&freeb, &totalb), "cudaMemGetInfo");
     // V as 32-byte records where the asked candidates fit with them, else packed:
     // neither the records nor the row kernels' copies make a launch hold fewer.
+    // Packed too where no row kernel writes it (k_atoms and k_force with rows of
+    // 166 slots, 64 candidates: 3695 us packed, 4041 with records).
     const size_t tables = sizeof(double) * (2 * (size_t)stride + ctx->pstride +
                                             (size_t)ctx->adj_ctas_max * stride * (1 + ADJ_WARPS) + (size_t)2048 * stride +
                                             2 * (size_t)ctx->P + 1);
     const size_t budget = (size_t)(0.6 * (double)(freeb + copies));
     const int cap = (int)std::min<size_t>(INT_MAX, std::max<size_t>(1, budget / (cand_bytes(3) + tables)));
     ctx->cand_cap = std::min(ctx->max_cand, cap);
-    d.vs = ctx->cand_cap * (cand_bytes(4) + tables) <= budget ? 4 : 3;
+    d.vs = ctx->rows_ok && ctx->cand_cap * (cand_bytes(4) + tables) <= budget ? 4 : 3;
     const size_t C = ctx->cand_cap;
     ctx->d_params = dalloc<double>(ctx, C * ctx->P);
     ctx->d_tabs = dalloc<double>(ctx, C * stride);

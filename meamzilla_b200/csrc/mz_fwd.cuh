@@ -646,6 +646,7 @@ __global__ void __launch_bounds__(BLOCK_SLOTS, JM ? 2 : sizeof(R) == 4 ? 4 : 3)
 // writes them without staging, 1408 -> 1200 us there and 1171 -> 1145 us for
 // 21 k atoms of 16 slots, 56 candidates).  Two candidates a thread gave 530 us
 // there, but 48 for 35 us with one candidate.  V is packed to 24 bytes where
+// the row kernels do not serve (spline5eq, rows of more than 128 slots), where
 // records would make a launch hold fewer candidates than were asked for, and
 // in the run without allocations, whose workspace the caller sized.
 constexpr int FORCE_LANES = 8;
