@@ -2113,11 +2113,8 @@ mz_status mz_gram_device(mz_ctx *ctx, int na, const double *d_a, int64_t lda, in
     const int64_t units = (n + unit - 1) / unit;
     const int Ti = (na + GRAM_T - 1) / GRAM_T, Tj = (nb + GRAM_T - 1) / GRAM_T;
     const int ntiles = vec ? 1 : (g.sym ? Tj * (Tj + 1) / 2 : Ti * Tj);
-    // the vector form: four CTAs per SM over the k ranges; the tiles: one (its
-    // eight warps keep the FP64 pipe busy, and fewer ranges leave fewer partials)
-    const int64_t per_sm = vec ? 4 : 1;
-    const int64_t want = std::max<int64_t>(1, per_sm * (int64_t)ctx->nsm / ntiles);
-    int64_t S = std::min(units, want);
+    // the vector form: four CTAs per SM over the k ranges
+    int64_t S = vec ? std::min<int64_t>(units, 4 * (int64_t)ctx->nsm) : gram_ranges(ntiles, units, (int64_t)na * nb, ctx->nsm);
     const int64_t per = (units + S - 1) / S;
     S = (units + per - 1) / per;  // no empty range
     g.S = (int)S;
@@ -2149,7 +2146,8 @@ mz_status mz_gram_device(mz_ctx *ctx, int na, const double *d_a, int64_t lda, in
     }
     ck(cudaGetLastError(), "k_gram");
     const int outs = na * nb;
-    k_gram_sum<<<(outs + 31) / 32, 1024, 0, ctx->stream>>>(g);
+    if (S <= GRAM_FEW) k_gram_sum_few<<<(outs + 255) / 256, 256, 0, ctx->stream>>>(g);
+    else k_gram_sum<<<(outs + 31) / 32, 1024, 0, ctx->stream>>>(g);
     ck(cudaGetLastError(), "k_gram_sum");
     ctx->launches += 2;
   });

@@ -23,19 +23,21 @@
 //                1024 k with B's chunk in shared memory, one warp per A row,
 //                lanes striding k, a fixed shuffle tree per row and chunk.
 //   k_gram_sum   a warp per run of partials, 32 outputs per CTA, the runs in
-//                order.
+//                order; k_gram_sum_few a thread per output.
 //
 // Bytes: k_gram_vec reads A once; k_gram_tile reads each 64-row block of A
 // once per output tile it takes part in (ceil(nb / 64) times in all).  The
 // vector form is HBM-bound, the square form bound by the FP64 pipe (a 64 x 64
 // tile costs an SM 4 cycles per 8 x 8 x 4 step).  The register-tile form
 // (4 x 4 per thread, 16 shared-memory wavefronts per 9 cycles of FMA, 510
-// partials added by one thread per output) took 116 us for 56 rows of 65 k
-// through the evaluator; this 52 (one or two CTAs per SM alike, three 56).
+// partials added by one thread per output) took 126 us for a call with 56 rows
+// of 65 k, from host to host; this 46 (one or two CTAs per SM alike, three 4 us
+// more).
 #pragma once
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 namespace mzb {
@@ -43,6 +45,7 @@ namespace mzb {
 constexpr int GRAM_T = 64;      // output tile edge of k_gram_tile
 constexpr int GRAM_BK = 32;     // k slice staged per step
 constexpr int GRAM_VEC = 4;     // largest nb served by k_gram_vec
+constexpr int GRAM_FEW = 32;    // ranges up to which k_gram_sum_few adds them
 constexpr int GRAM_VK = 1024;   // k chunk of k_gram_vec
 
 struct GramArgs {
@@ -247,22 +250,27 @@ __global__ void __launch_bounds__(256) k_gram_vec(GramArgs g) {
   }
 }
 
+// where output t's partials start: of its mirror where only that was computed
+__device__ __forceinline__ const double *gram_partials(const GramArgs &g, int t) {
+  int i = t / g.nb, j = t % g.nb;
+  if (g.sym && j < i) {
+    const int x = i;
+    i = j;
+    j = x;
+  }
+  return g.partial + (size_t)i * g.nb + j;
+}
+
+// Many ranges (few outputs)
 __global__ void __launch_bounds__(1024) k_gram_sum(GramArgs g) {
   __shared__ double part[32][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x * 32 + lane, outs = g.na * g.nb;
   const int per = (g.S + 31) / 32, s1 = min(g.S, (warp + 1) * per);
   double v = 0.0;
   if (t < outs) {
-    int i = t / g.nb, j = t % g.nb;
-    if (g.sym && j < i) {  // its mirror was computed
-      const int x = i;
-      i = j;
-      j = x;
-    }
-    const double *p = g.partial + (size_t)i * g.nb + j;
-    const size_t stride = (size_t)outs;
+    const double *p = gram_partials(g, t);
 #pragma unroll 8
-    for (int s = warp * per; s < s1; ++s) v += p[s * stride];
+    for (int s = warp * per; s < s1; ++s) v += p[(size_t)s * outs];
   }
   part[warp][lane] = v;
   __syncthreads();
@@ -272,6 +280,41 @@ __global__ void __launch_bounds__(1024) k_gram_sum(GramArgs g) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   const int q = blockIdx.x * 32 + warp;
   if (lane == 0 && q < outs) g.out[q] = v;
+}
+
+// Few ranges, many outputs: a thread per output.  (A CTA of 1024 threads per 32
+// outputs made 1000 rows of 5000, one range, a call of 382 us; this 256.)
+__global__ void __launch_bounds__(256) k_gram_sum_few(GramArgs g) {
+  const int t = blockIdx.x * 256 + threadIdx.x, outs = g.na * g.nb;
+  if (t >= outs) return;
+  const double *p = gram_partials(g, t);
+  double v = 0.0;
+#pragma unroll 8
+  for (int s = 0; s < g.S; ++s) v += p[(size_t)s * outs];
+  g.out[t] = v;
+}
+
+// Ranges of k that k_gram_tile's `ntiles` tiles are cut into: an SM runs one
+// CTA at a time (eight warps keep its FP64 pipe busy), so the time is that of
+// ceil(ntiles S / nsm) rounds of ceil(units / S) slices, plus about three
+// slices a round for the pipeline's start and the partials' store, plus
+// reading the partials back (a slice takes 1.55 us).  At most four CTAs' worth
+// of ranges per SM, which bounds the workspace.  With nsm / ntiles ranges
+// 760 rows of 5000 (78 tiles, one range) took 326 us on half of the SMs and
+// 1200 rows (190 tiles, a short second round) 677; this rule 166 and 350.
+inline int64_t gram_ranges(int64_t ntiles, int64_t units, int64_t outs, int nsm) {
+  const int64_t most = std::min(units, (4 * (int64_t)nsm + ntiles - 1) / ntiles);
+  int64_t best = 1;
+  double t = 1e300;
+  for (int64_t rounds = (ntiles + nsm - 1) / nsm, S = 0; S < most; ++rounds) {
+    S = std::min(most, rounds * nsm / ntiles);  // the most ranges in this many rounds
+    const double x = rounds * ((double)((units + S - 1) / S) + 3.0) + 2.6e-6 * (double)(S * outs);
+    if (x < t) {
+      t = x;
+      best = S;
+    }
+  }
+  return best;
 }
 
 }  // namespace mzb
