@@ -199,6 +199,7 @@ struct mz_ctx {
   struct Tune {
     bool done = false;
     bool fm = false;  // mixed meam/spline: the triplet-moment path
+    bool rows_timed = true;  // the rest was timed (not where the moment path made that needless)
     int fwd = 0, adj = 0, ctas = 0;
     int nc = 1;      // candidates per CTA of the forward (2: k_atoms2, mixed meam/spline)
     int adj_nc = 1;  // candidates per CTA of the adjoint (2: k_adj2)
@@ -1220,7 +1221,8 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
   if (!t.done) {
     const std::vector<int64_t> key = {ctx->device,     ctx->natoms,    ctx->npairs, ctx->ncells, ctx->pot.style,
                                       ctx->pot.ntypes, ctx->P,         precision,   grad,        ctx->q5,
-                                      ctx->autotune,   ctx->nblk[0],   ctx->nadjblk[0], ctx->fm_mode};
+                                      ctx->autotune,   ctx->nblk[0],   ctx->nadjblk[0], ctx->fm_mode,
+                                      ctx->rows_ok,    ctx->radj.ready};
     bool cached = false;
     mz_ctx::Tune best;
     {
@@ -1244,12 +1246,22 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
       apply_variant(ctx, best);
       return;
     }
-    if (cached && best.fm && !fm_prepare(ctx)) best.fm = false;
+    if (cached && best.fm && !fm_prepare(ctx)) {  // no memory for it here: the row kernels' own choice
+      best.fm = false;
+      if (!best.rows_timed) {
+        cached = false;
+        best = mz_ctx::Tune{};
+        best.ctas = adj_ctas_for(ctx, 0, ctx->adj_per_sm);
+      }
+    }
     if (!cached) {
       // the FP64 row kernels have no variants to time
-      bool fixed = precision == MZ_FP64 && ctx->rows_ok && (!grad || ctx->radj.ready);
+      const bool fwd_fixed = precision == MZ_FP64 && ctx->rows_ok;
+      bool fixed = fwd_fixed && (!grad || ctx->radj.ready);
       // Nor are the mixed row kernels' worth timing where the moment path beats
-      // their first variant by half: their best one is within 30 % of it, and
+      // their first variant by half: over 108 shapes of 1 to 3 species, rows of
+      // 26 to 96 slots, 1 to 128 candidates, with and without the gradient,
+      // the first variant's call took at most 1.32 times their best one's, and
       // the 18 trials of a large launch take seconds.
       if (precision == MZ_MIXED && ctx->autotune == 1 && ctx->fm.eligible && ctx->fm_mode == 1 && fm_prepare(ctx)) {
         const int64_t l0 = ctx->launches;
@@ -1263,6 +1275,7 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
         }
         ctx->launches = l0;
         best.fm = 1.5 * t[1] < t[0];
+        best.rows_timed = !best.fm;
         fixed = best.fm;
       }
       if (ctx->autotune == 1 && !fixed) {
@@ -1271,7 +1284,7 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
         trial(ctx, n, d_params, precision, grad, MZ_K_ATOMS);  // warm-up
         double bt = 1e300;
         const int ncs = (precision == MZ_MIXED && ctx->nc2_ok && n > 1) ? 2 : 1;
-        for (int nc = 1; nc <= ncs; ++nc)
+        for (int nc = 1; nc <= ncs && !fwd_fixed; ++nc)
           for (int v = 0; v < mz_ctx::NCAPS; ++v) {
             mz_ctx::Tune c = best;
             c.fwd = v;
@@ -1332,7 +1345,15 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
       }
       best.done = true;
       std::lock_guard<std::mutex> lk(g_tune_mu);
-      g_tune_cache.emplace(key, best);
+      auto &kept = g_tune_cache.emplace(key, best).first->second;
+      if (!kept.rows_timed && best.rows_timed) {  // complete it; contexts with room keep the moment path
+        kept.fwd = best.fwd;
+        kept.adj = best.adj;
+        kept.ctas = best.ctas;
+        kept.nc = best.nc;
+        kept.adj_nc = best.adj_nc;
+        kept.rows_timed = true;
+      }
     }
     t = best;
     t.done = true;
