@@ -515,7 +515,12 @@ __global__ void __launch_bounds__(32 * ROWS_W, JM ? 3 : 4)
           if (JM) V[k] += Vd[s][k];
           q[k] += V[k];
         }
-        store_vec(Vc + vs * (int64_t)p, vs, V[0], V[1], V[2]);
+        if (vs == 4) {
+          store_vec4(Vc + 4 * (int64_t)p, V[0], V[1], V[2]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 3; ++k) Vc[3 * (int64_t)p + k] = V[k];
+        }
         const double r = KEEP ? rk[s] : uzr[lo + p].y, x = V[0] * r, y = V[1] * r, z = V[2] * r;
         q[4] -= u[s][0] * x;
         q[5] -= u[s][1] * y;
