@@ -343,7 +343,7 @@ mz_status mz_tuning(mz_ctx *ctx, int precision, int grad, int *choice);
 enum {
   MZ_K_PREP = 0,    /* coefficients -> knot and evaluation tables          */
   MZ_K_ATOMS,       /* densities, embedding, per-slot reaction vectors      */
-  MZ_K_GATHER,      /* per-atom forces, force residuals                     */
+  MZ_K_GATHER,      /* per-atom forces, force residuals (k_force)           */
   MZ_K_CELLS,       /* per-cell energy, stress, residual entries, objective */
   MZ_K_FINAL,       /* sum of squares + punishments (moment path)           */
   MZ_K_ADJ,         /* adjoint pass over the neighbour rows                 */
@@ -357,6 +357,10 @@ enum {
   MZ_K_FM_GRAD,     /* moment-space and B-spline gradients -> knot table    */
   MZ_K_GRAD_SUM,    /* table-gradient partials summed (row kernels)         */
   MZ_K_RADIAL,      /* radial functions' gradient sums (FP64 row kernels)   */
+  /* the FP64 row kernels' counterparts of MZ_K_ATOMS, _ADJ and _GRAD_FINAL   */
+  MZ_K_ROWS,
+  MZ_K_ROWS_ADJ,
+  MZ_K_ROWS_GRAD_FINAL,
   MZ_NKERNELS
 };
 const char *mz_kernel_name(int kernel);

@@ -134,7 +134,7 @@ _SIGS = {
                                        C.c_void_p]),
 }
 
-MZ_NKERNELS = 15
+MZ_NKERNELS = 18
 
 
 def lib() -> C.CDLL:

@@ -592,7 +592,7 @@ void enqueue_rows_adj(mz_ctx *ctx, int n, double *d_grad) {
   a.W1 = ctx->d_V;
   a.stream = ctx->stream;
   {
-    Bracket b(ctx, MZ_K_ADJ);
+    Bracket b(ctx, MZ_K_ROWS_ADJ);
     ck(rows_adjoint(a), "k_rows_adj launch");
   }
   {
@@ -609,7 +609,7 @@ void enqueue_rows_adj(mz_ctx *ctx, int n, double *d_grad) {
   g.nparts[1] = a.rctas;
   g.len[1] = 4 * a.radial.nb;
   launch_grad_sum(ctx, n, g);
-  Bracket b(ctx, MZ_K_GRAD_FINAL);
+  Bracket b(ctx, MZ_K_ROWS_GRAD_FINAL);
   k_rows_grad_final<<<n, 256, 2 * sizeof(double) * ctx->stride, ctx->stream>>>(
       ctx->pot, a.radial, ra.nang, ctx->d_geom, ctx->d_tabs, ra.sum, ra.rsum, ctx->d_M, ctx->d_cmap, ctx->P, d_grad);
   ck(cudaGetLastError(), "k_rows_grad_final launch");
@@ -888,9 +888,10 @@ void enqueue(mz_ctx *ctx, int n, const double *d_params, int precision, double *
     return;
   }
   {
-    Bracket b(ctx, MZ_K_ATOMS);
+    const bool rows = !mixed && ctx->rows_ok;
+    Bracket b(ctx, rows ? MZ_K_ROWS : MZ_K_ATOMS);
     const size_t sa = ctx->smem_atoms[mixed ? 1 : 0];
-    if (!mixed && ctx->rows_ok) {
+    if (rows) {
       RowsForward a{ctx->db,     ctx->pot,     meam,       ctx->max_row, n,
                     ctx->nsm,    ctx->smem_optin, ctx->d_geom, ctx->d_tabs, ctx->d_ptabs,
                     ctx->d_V,    ctx->d_aout,  grad && meam ? ctx->d_aux : nullptr, st};
@@ -2177,8 +2178,8 @@ mz_status mz_gram_device(mz_ctx *ctx, int na, const double *d_a, int64_t lda, in
 const char *mz_kernel_name(int k) {
   static const char *names[MZ_NKERNELS] = {"k_prep",   "k_atoms",      "k_force",   "k_cells",  "k_final",
                                            "k_adj",    "k_grad_final", "k_fm_coef", "k_fm_fwd", "k_fm_epi",
-                                           "k_fm_pre", "k_fm_adj",     "k_fm_grad",    "k_grad_sum",
-                                           "k_rows_radial"};
+                                           "k_fm_pre", "k_fm_adj",     "k_fm_grad", "k_grad_sum",
+                                           "k_rows_radial", "k_rows",  "k_rows_adj", "k_rows_grad_final"};
   return (k >= 0 && k < MZ_NKERNELS) ? names[k] : "?";
 }
 
