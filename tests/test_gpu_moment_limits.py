@@ -1,0 +1,31 @@
+"""Mixed-precision meam where the moment path's tables are at and beyond the
+device's shared memory (U of 64 knots, two species; 224 to 242 KB of 227):
+the calls run, on the row kernels where they do not fit, within the mixed
+precision bars of the parity tests (objective 1e-6, forces 1e-5 of the largest
+one or of 1 eV/A)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nu,nr", [(64, 9), (64, 10), (64, 11), (64, 12), (64, 13), (60, 14)])
+def test_mixed_calls_near_the_limit(nu, nr):
+    from meamzilla_b200 import synth
+    from meamzilla_b200.potential import MZ_FP64, MZ_MIXED, Database, Evaluator, PotentialFile
+    spec = synth.in_range_variant(synth.teacher_potential("meam/spline", 2, 4.3, seed=2))
+    for i, group in enumerate(spec.groups):
+        for s in group:
+            n = {0: nr, 1: nr, 2: nu, 3: nr, 4: 8}[i]
+            s.y = np.interp(np.linspace(s.left, s.right, n), np.linspace(s.left, s.right, s.nknots), s.y)
+    pot = PotentialFile.from_spec(spec)
+    rng = np.random.default_rng(6)
+    cells = synth.make_cells(30, lambda r: 60, rng, ntypes=2)
+    for c in cells:
+        c.force0 = rng.normal(0, 0.3, c.force0.shape)
+    ev = Evaluator(Database.from_cells(cells, pot), pot, 1.0, 1.0, 0, max_candidates=64)
+    X = synth.perturbed(pot.coeffs(), 64, 0.01, seed=5)
+    a, b = ev.objective(X, MZ_FP64, forces=True), ev.objective(X, MZ_MIXED, forces=True)
+    assert np.all(np.abs(a["obj"] - b["obj"]) <= 1e-6 * a["obj"])
+    assert np.max(np.abs(a["forces"] - b["forces"])) <= 1e-5 * max(1.0, np.max(np.abs(a["forces"])))
+    ev.objective_grad(X[:2], MZ_MIXED)
