@@ -72,9 +72,15 @@ def build(force: bool = False, verbose: bool = False) -> str:
             print(" ".join(cmd), flush=True)
         running.append((cmd, subprocess.Popen(cmd)))  # side by side
         objs.append(obj)
-    for cmd, p in running:
-        if p.wait() != 0:
-            raise subprocess.CalledProcessError(p.returncode, cmd)
+    try:
+        failed = [(p.returncode, cmd) for cmd, p in running if p.wait() != 0]  # every compiler has ended
+    finally:
+        for _, p in running:
+            if p.poll() is None:
+                p.kill()
+                p.wait()
+    if failed:
+        raise subprocess.CalledProcessError(*failed[0])
     tmp = LIB + ".tmp"
     subprocess.run([nvcc()] + ARCH + ["-shared", "-o", tmp] + objs + ["-lcudart"], check=True)
     os.replace(tmp, LIB)
