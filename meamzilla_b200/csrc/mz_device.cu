@@ -498,7 +498,8 @@ void launch_grad_final(mz_ctx *ctx, int n, int nparts, double *d_grad) {
 bool rows_adj_prepare(mz_ctx *ctx) {
   auto &ra = ctx->radj;
   if (ra.ready) return true;
-  if (ra.failed || !ctx->rows_ok || ctx->pot.nj > 0) return false;
+  ra.failed = ra.failed || !ctx->rows_ok || ctx->pot.nj > 0;
+  if (ra.failed) return false;
   const bool meam = style_meam(ctx->pot.style);
   const int N = ctx->natoms;
   const size_t C = ctx->cand_cap, Np = ctx->npairs;
@@ -1219,11 +1220,16 @@ double trial(mz_ctx *ctx, int n, const double *d_params, int precision, bool gra
 // a call that finds no choice made runs the first variant (FP64 gradients the
 // block kernels, mixed calls the row kernels), and the choice is left open.
 void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, bool grad) {
+  mz_ctx::Tune &t = ctx->tune[precision][grad ? 1 : 0];
+  const bool adj_plan = precision == MZ_FP64 && grad && !ctx->radj.ready && !ctx->radj.failed;
+  if (t.done && !adj_plan) {
+    apply_variant(ctx, t);
+    return;
+  }
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   ck(cudaStreamIsCapturing(ctx->stream, &status), "capture status");
   const bool capturing = status != cudaStreamCaptureStatusNone;
-  if (precision == MZ_FP64 && grad && !capturing) rows_adj_prepare(ctx);
-  mz_ctx::Tune &t = ctx->tune[precision][grad ? 1 : 0];
+  if (adj_plan && !capturing) rows_adj_prepare(ctx);
   if (!t.done) {
     const std::vector<int64_t> key = {ctx->device,     ctx->natoms,    ctx->npairs, ctx->ncells, ctx->pot.style,
                                       ctx->pot.ntypes, ctx->P,         precision,   grad,        ctx->q5,
@@ -1265,9 +1271,9 @@ void tune_variant(mz_ctx *ctx, int n, const double *d_params, int precision, boo
       const bool fwd_fixed = precision == MZ_FP64 && ctx->rows_ok;
       bool fixed = fwd_fixed && (!grad || ctx->radj.ready);
       // Nor are the mixed row kernels' worth timing where the moment path beats
-      // their first variant by half: over 108 shapes of 1 to 3 species, rows of
+      // their first variant by half: over 96 calls of 1 and 2 species, rows of
       // 26 to 96 slots, 1 to 128 candidates, with and without the gradient,
-      // the first variant's call took at most 1.32 times their best one's, and
+      // the first variant's took at most 1.32 times their best one's time, and
       // the 18 trials of a large launch take seconds.
       if (precision == MZ_MIXED && ctx->autotune == 1 && ctx->fm.eligible && ctx->fm_mode == 1 && fm_prepare(ctx)) {
         const int64_t l0 = ctx->launches;

@@ -20,7 +20,7 @@
 // summed, and a lane's slots advance side by side (the FP64 pipe takes 1.8
 // instructions a clock from warps with four independent chains, 1.25 from
 // any number of warps with one).  Measured (k_atoms -> k_rows): 84 k atoms of
-// 41 slots, 1 candidate 581 -> 379 us (shared memory 71 %, FP64 52 %); 21 k
+// 41 slots, 1 candidate 581 -> 378 us (L1 and shared memory 70 %, FP64 52 %); 21 k
 // atoms of 16 slots, 56 candidates 2397 -> 1145 us; EAM, 18 k atoms of 42
 // slots, 128 candidates 4811 -> 1200 us.
 #pragma once
@@ -160,7 +160,7 @@ __device__ __forceinline__ int rows_knot(double c, const RowSpl &g, double &b) {
 // s0 can meet itself, so one comparison and select per partner does it (MEAM,
 // 21 k atoms of 16 slots, 56 candidates: 1381 us a call).  Without, every slot
 // compares, in one loop: for JMEAM, whose passes would otherwise be four loops
-// each (12 k atoms, 16 candidates: 573 us a call, in runs 603).
+// each (10 k atoms, 16 candidates: 573 us a call, in runs 603).
 // CL: knots that do not cover the cosines -- the interval is clamped, and a
 // partner beyond the upper cut is no triplet.
 template <bool CL, int NS, int SPL, int LPA, bool GM, bool RUNS, class W>

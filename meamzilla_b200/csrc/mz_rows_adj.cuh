@@ -11,7 +11,7 @@
 //   lane's own (shared memory, power basis about the interval's middle);
 // - k_rows_radial sums the radial gradients: which interval of which spline a
 //   slot falls into does not depend on the candidate, so the slots of every
-//   segment (512 to 2048) are sorted by it once (k_rows_sort), and a warp adds
+//   segment (256 to 2048) are sorted by it once (k_rows_sort), and a warp adds
 //   up one bucket in registers;
 // - both leave partials in an order fixed by the database, summed in order by
 //   k_grad_sum: the gradient is bit-identical from call to call.
