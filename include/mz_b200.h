@@ -320,8 +320,8 @@ mz_status mz_launch_count(const mz_ctx *ctx, int64_t *launches);
 mz_status mz_tensor_core_forward(const mz_ctx *ctx, int *on);
 
 /* Launch variants chosen by the context's autotuner (no reference
- * counterpart).  FP64 calls on the row kernels have none.  Otherwise the
- * first objective call of a precision, with or without the gradient, times on the caller's own candidates the forward kernel at
+ * counterpart).  FP64 calls on the row kernels have none (a jmeam gradient
+ * has the adjoint's).  Otherwise the first objective call of a precision, with or without the gradient, times on the caller's own candidates the forward kernel at
  * three atom-block sizes (blocks of at most 256, 192 or 128 pair slots, a
  * quarter as many atoms) and, for the gradient, the adjoint at the same three
  * sizes and two persistent-grid sizes, and keeps the fastest for the
