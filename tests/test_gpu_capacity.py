@@ -12,8 +12,27 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture()
+def short_memory():
+    """Fills device memory up to 12 GB; freed again whatever the test does."""
+    import torch
+    held = []
+
+    def fill():
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        held.append(torch.empty(max(1, torch.cuda.mem_get_info()[0] - (12 << 30)), dtype=torch.uint8, device="cuda"))
+
+    def free():
+        held.clear()
+        torch.cuda.empty_cache()
+
+    yield fill, free
+    free()
+
+
 @pytest.mark.parametrize("style", ["eam/spline", "meam/spline"])
-def test_candidates_per_launch_when_memory_binds(style):
+def test_candidates_per_launch_when_memory_binds(style, short_memory):
     import torch
     from meamzilla_b200 import synth
     from meamzilla_b200._lib import check, lib
@@ -29,9 +48,8 @@ def test_candidates_per_launch_when_memory_binds(style):
              for _ in range(400 if meam else 1600)]
     db = Database.from_cells(cells, pot, device=0)
     stats = db.stats()
-    torch.cuda.synchronize()
-    torch.cuda.empty_cache()
-    filler = torch.empty(max(1, torch.cuda.mem_get_info()[0] - (12 << 30)), dtype=torch.uint8, device="cuda")
+    fill, unfill = short_memory
+    fill()
     free = torch.cuda.mem_get_info()[0]
     ev = Evaluator(db, pot, 1.0, 1.0, 0, max_candidates=100000)
     one = torch.zeros(1, dtype=torch.float64, device="cuda")
@@ -59,8 +77,8 @@ def test_candidates_per_launch_when_memory_binds(style):
     ev.objective_grad_device(x, obj, grad, MZ_FP64)
     ev.sync()
     obj, E, grad, mixed = (t.cpu().numpy() for t in (obj, E, grad, mixed))
-    del ev, filler, x, one
-    torch.cuda.empty_cache()
+    del ev, x, one
+    unfill()
     ref = Evaluator(db, pot, 1.0, 1.0, 0, max_candidates=2)
     for c in (0, n // 2, n - 1):
         r = ref.objective(X[c:c + 1], MZ_FP64, errvec=True)

@@ -48,9 +48,13 @@ def test_row_variant_where_the_moment_path_does_not_fit():
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     filler = torch.empty(torch.cuda.mem_get_info()[0] - (600 << 20), dtype=torch.uint8, device="cuda")
-    second = Evaluator(db, pot, 1.0, 1.0, 0, max_candidates=64)
-    got = second.objective(X[:8], MZ_MIXED)
-    assert second.moment_path(MZ_MIXED, False) == 0
+    try:
+        second = Evaluator(db, pot, 1.0, 1.0, 0, max_candidates=64)
+        got = second.objective(X[:8], MZ_MIXED)
+        on, tuning = second.moment_path(MZ_MIXED, False), second.tuning(MZ_MIXED, False)
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert on == 0
     assert np.all(np.abs(got - obj[:8]) <= 1e-6 * np.abs(got))
-    assert second.tuning(MZ_MIXED, False)["forward_candidates_per_cta"] == 2
-    del filler
+    assert tuning["forward_candidates_per_cta"] == 2
