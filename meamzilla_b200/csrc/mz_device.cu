@@ -1793,7 +1793,7 @@ mz_status mz_create(const mz_db *dbh, const mz_pot *poth, const mz_settings *set
           if (s < dp.s_U || s >= dp.s_f) PB = std::max(PB, pot.spline(s).nknots + 2);
         for (int s = 0; s < dp.s_g; ++s)
           if (s < dp.s_U || s >= dp.s_f) NBp = std::max(NBp, pot.spline(s).nknots + 2);
-        if (pot.ntypes * NA <= 32 && NN <= FM_MAXN && PB <= 23 && db.max_row <= BLOCK_SLOTS) {
+        if (Np > 0 && pot.ntypes * NA <= 32 && NN <= FM_MAXN && PB <= 23 && db.max_row <= BLOCK_SLOTS) {
           FmPlan &fp = ctx->fm.plan;
           fp.nt = pot.ntypes;
           fp.NA = NA;

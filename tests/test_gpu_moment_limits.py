@@ -29,3 +29,21 @@ def test_mixed_calls_near_the_limit(nu, nr):
     assert np.all(np.abs(a["obj"] - b["obj"]) <= 1e-6 * a["obj"])
     assert np.max(np.abs(a["forces"] - b["forces"])) <= 1e-5 * max(1.0, np.max(np.abs(a["forces"])))
     ev.objective_grad(X[:2], MZ_MIXED)
+
+
+def test_mixed_calls_without_pairs():
+    """Isolated atoms alone: nothing to contract, the row kernels serve."""
+    from meamzilla_b200 import synth
+    from meamzilla_b200.potential import MZ_FP64, MZ_MIXED, Database, Evaluator, PotentialFile
+    rng = np.random.default_rng(3)
+    cells = [synth.Cell(lattice=np.eye(3) * 30.0, types=np.zeros(1, dtype=int), pos=np.zeros((1, 3)),
+                        force0=rng.normal(0, 0.3, (1, 3)), energy0=-1.0, stress0=rng.normal(0, 1e-3, 6)) for _ in range(5)]
+    pot = PotentialFile.from_spec(synth.in_range_variant(synth.teacher_potential("meam/spline", 1, 4.3, seed=2)))
+    db = Database.from_cells(cells, pot)
+    assert db.stats()["npairs"] == 0
+    ev = Evaluator(db, pot, 1.0, 1.0, 0, max_candidates=3)
+    X = synth.perturbed(pot.coeffs(), 3, 0.01, seed=5)
+    a, b = ev.objective_grad(X, MZ_FP64), ev.objective_grad(X, MZ_MIXED)
+    assert np.all(np.abs(a[0] - b[0]) <= 1e-6 * a[0])
+    assert np.max(np.abs(a[1] - b[1])) <= 1e-4 * np.max(np.abs(a[1]))
+    assert np.all(np.abs(ev.objective(X, MZ_MIXED) - a[0]) <= 1e-6 * a[0])
