@@ -761,8 +761,10 @@ bool fm_prepare(mz_ctx *ctx) {
   smem_attr(k_fm_gemm_fwd<8>, fm_fwd_smem<8>(fp.Dpad));
   smem_attr(k_fm_epi<0>, fm_epi_smem(ctx->nsplines, fp.nt, fp.NB, 64));
   smem_attr(k_fm_epi<64>, fm_epi_smem(ctx->nsplines, fp.nt, fp.NB, 64));
-  smem_attr(k_fm_gemm_adj<false>, fm_adj_smem(fp.Dpad, 64));
-  if (fm.tc8) smem_attr(k_fm_gemm_adj<true>, fm_adj_smem(fp.Dpad, 64, true));
+  smem_attr(k_fm_gemm_adj<false, 256>, fm_adj_smem(fp.Dpad, 64));
+  smem_attr(k_fm_gemm_adj<false, FM_ADJ_MAXT>, fm_adj_smem(fp.Dpad, 64));
+  if (fm.tc8) smem_attr(k_fm_gemm_adj<true, 256>, fm_adj_smem(fp.Dpad, 64, true));
+  if (fm.tc8) smem_attr(k_fm_gemm_adj<true, FM_ADJ_MAXT>, fm_adj_smem(fp.Dpad, 64, true));
   fm.ready = true;
   return true;
 }
@@ -852,13 +854,14 @@ void enqueue_fm(mz_ctx *ctx, int n, double *d_obj, double *d_errvec, double *d_f
   }
   {
     Bracket b(ctx, MZ_K_FM_ADJ);
-    const int threads = ((fp.Dpad / FM_ROWS) * (CG / 8) + 31) / 32 * 32;
     if (ctx->fm.tc8a) {
       k_fm_gemm_adj8<<<dim3(fp.nctas_adj, G), FM8_ATHREADS, fm8_adj_smem(), st>>>(fp, n, ctx->d_err);
-    } else if (ctx->fm.tc8)
-      k_fm_gemm_adj<true><<<dim3(fp.nctas_adj, G), std::min(threads, 256), fm_adj_smem(fp.Dpad, CG, true), st>>>(fp);
-    else
-      k_fm_gemm_adj<false><<<dim3(fp.nctas_adj, G), std::min(threads, 256), fm_adj_smem(fp.Dpad, CG), st>>>(fp);
+    } else {
+      const int threads = fm_adj_threads(fp.Dpad, CG);
+      auto adj = ctx->fm.tc8 ? (threads <= 256 ? k_fm_gemm_adj<true, 256> : k_fm_gemm_adj<true, FM_ADJ_MAXT>)
+                             : (threads <= 256 ? k_fm_gemm_adj<false, 256> : k_fm_gemm_adj<false, FM_ADJ_MAXT>);
+      adj<<<dim3(fp.nctas_adj, G), threads, fm_adj_smem(fp.Dpad, CG, ctx->fm.tc8), st>>>(fp);
+    }
     ck(cudaGetLastError(), "k_fm_gemm_adj launch");
   }
   {

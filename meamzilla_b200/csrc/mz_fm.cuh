@@ -1239,8 +1239,14 @@ __host__ __device__ inline size_t fm_adj_smem(int Dpad, int CG, bool dig8 = fals
          (dig8 ? (size_t)FM8_SUBRAW + sizeof(double) * 3 * FM_SUB : 0);
 }
 
-template <bool DIG8>
-__global__ void __launch_bounds__(256, 1) k_fm_gemm_adj(FmPlan fp) {
+// MT: the block's threads at most.  A thread takes FM_ROWS features and 8
+// candidates, so more than 256 features a type need more than 256 threads for
+// 64 candidates (fm_adj_threads).
+inline int fm_adj_threads(int Dpad, int CG) { return ((Dpad / FM_ROWS) * (CG / 8) + 31) / 32 * 32; }
+constexpr int FM_ADJ_MAXT = 512;
+
+template <bool DIG8, int MT>
+__global__ void __launch_bounds__(MT, 1) k_fm_gemm_adj(FmPlan fp) {
   extern __shared__ __align__(16) float asm_[];
   const int CG = fp.CG, gy = blockIdx.y;
   const size_t xsz = (size_t)3 * fp.Dpad * FM_XS, ysz = (size_t)FM_SUB * 3 * CG;
@@ -1303,10 +1309,10 @@ __global__ void __launch_bounds__(256, 1) k_fm_gemm_adj(FmPlan fp) {
       const int j = i % FM_SUB, d4 = (i / FM_SUB) % nd4, t = i / (FM_SUB * nd4);
       const int d = 4 * d4, kb = d >> 7;
       const uint32_t o = sw128_byte(j, d & 127);
-      uint32_t w[FM8_DIG];
+      uint32_t w[FM8_DIG] = {};
 #pragma unroll
-      for (int l = 0; l < FM8_DIG; ++l)
-        w[l] = *reinterpret_cast<const uint32_t *>(raw + (size_t)((t * 2 + kb) * FM8_DIG + l) * 2048 + o);
+      for (int l = 0; l < FM8_DIG; ++l)  // Dpad can exceed the FM8_D features that have digits: zero
+        if (d < FM8_D) w[l] = *reinterpret_cast<const uint32_t *>(raw + (size_t)((t * 2 + kb) * FM8_DIG + l) * 2048 + o);
       const double sc = rsc[t * FM_SUB + j];
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
