@@ -649,8 +649,10 @@ bool fm_prepare(mz_ctx *ctx) {
   // second wave would run a fixed share of the blocks on a half-empty GPU);
   // launches of fewer candidates stage less and stay resident as well
   fm.smem_pre = fm_pre_smem(ctx->nsplines, 64, fp.nt, fp.NB, fp.ustride);
-  // many knots of U or of the radial functions: the row kernels serve
-  if (std::max(fm.smem_pre, fm_epi_smem(ctx->nsplines, fp.nt, fp.NB, 64)) > (size_t)ctx->smem_optin) {
+  // many knots (of U, of the radial functions, of f and g together): the row kernels serve
+  if (std::max({fm.smem_pre, fm_epi_smem(ctx->nsplines, fp.nt, fp.NB, 64), fm_adj_smem(fp.Dpad, 64)}) >
+          (size_t)ctx->smem_optin ||
+      fm_adj_threads(fp.Dpad, 64) > FM_ADJ_MAXT) {
     fm.failed = true;
     return false;
   }
